@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import unittest
 
 import numpy as np
 
@@ -23,11 +24,15 @@ class RefError(RuntimeError):
         self.identifier = ident
 
 
+class RefMissing(FileNotFoundError, unittest.SkipTest):
+    """The reference's sources were not there to build: a comparison with it is skipped."""
+
+
 class RefMex:
     def __init__(self, name):
         path = os.path.join(REF_DIR, name + ".so")
         if not os.path.exists(path):
-            raise FileNotFoundError(path + " (build with: make -C oracle)")
+            raise RefMissing(path + " (build with: make -C oracle)")
         L = C.CDLL(path)
         L.fm_numeric.restype = C.c_void_p
         L.fm_numeric.argtypes = [C.c_int, C.c_int, C.POINTER(C.c_size_t), C.c_void_p, C.c_void_p]
