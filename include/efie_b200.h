@@ -411,6 +411,14 @@ void efie_debug_set_selftest_tiles(int tile_chain, int tile_bulk, int resident);
  * than one batch), process-wide.  No counterpart in the reference. */
 void efie_debug_disable_warm_start(int disable);
 
+/* Z of nf (at most the plan's batch) frequencies as a sweep assembles them
+ * from frequency-independent moments, Z[nf][Ne x Ne] column-major on the
+ * host; `tiles` > 0 limits the 32 x 32 entry tiles held at a time.  *terms:
+ * the series' terms, 0 when it does not serve these frequencies (Z is then
+ * left alone).  No counterpart in the reference. */
+efie_status efie_debug_plan_series(efie_plan *plan, const double *freqs, int32_t nf, int32_t tiles, int32_t *terms,
+                                   efie_c128 *Z);
+
 /* ---------------------------------------------------------------------- */
 /* Centroid assembly without device allocation                             */
 /* ---------------------------------------------------------------------- */

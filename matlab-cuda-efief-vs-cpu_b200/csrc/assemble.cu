@@ -18,10 +18,9 @@
 #include <vector>
 
 #include "efie_internal.h"
+#include "quad.cuh"
 
 namespace {
-
-constexpr double kPi = 3.141592653589793238462643383279502884;
 
 struct Mom {
     double v[16];  // S0(re,im) S1x S1y S1z S2x S2y S2z S3 (re,im each)
@@ -593,50 +592,6 @@ __global__ void __launch_bounds__(64) k_self_moments_mf(int Nt, bool sym, int P,
 // Wilton et al. 1984 / Graglia 1993) at every outer rule point, the smooth
 // part with the rule on both triangles.  One warp per pair (t1 <= t2).
 // ---------------------------------------------------------------------------
-// I0 = int_T 1/R dS', J = int_T (r' - r)/R dS' for triangle (a0, a1, a2).
-__device__ void potential_integrals(const double3 a0, const double3 a1, const double3 a2, const double3 r,
-                                    double &I0, double3 &J) {
-    const double3 A[3] = {a0, a1, a2};
-    double3 n = make_double3((a1.y - a0.y) * (a2.z - a0.z) - (a1.z - a0.z) * (a2.y - a0.y),
-                             (a1.z - a0.z) * (a2.x - a0.x) - (a1.x - a0.x) * (a2.z - a0.z),
-                             (a1.x - a0.x) * (a2.y - a0.y) - (a1.y - a0.y) * (a2.x - a0.x));
-    const double nn = sqrt(n.x * n.x + n.y * n.y + n.z * n.z);
-    n.x /= nn; n.y /= nn; n.z /= nn;
-    const double d = n.x * (r.x - a0.x) + n.y * (r.y - a0.y) + n.z * (r.z - a0.z);
-    const double ad = fabs(d);
-    const double3 rho = make_double3(r.x - d * n.x, r.y - d * n.y, r.z - d * n.z);
-    double s0 = 0.0, vx = 0.0, vy = 0.0, vz = 0.0;
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-        const double3 p = A[i], q = A[(i + 1) % 3];
-        double3 l = make_double3(q.x - p.x, q.y - p.y, q.z - p.z);
-        const double ll = sqrt(l.x * l.x + l.y * l.y + l.z * l.z);
-        l.x /= ll; l.y /= ll; l.z /= ll;
-        const double3 u = make_double3(l.y * n.z - l.z * n.y, l.z * n.x - l.x * n.z, l.x * n.y - l.y * n.x);
-        const double P0 = (p.x - rho.x) * u.x + (p.y - rho.y) * u.y + (p.z - rho.z) * u.z;
-        const double lp = (q.x - rho.x) * l.x + (q.y - rho.y) * l.y + (q.z - rho.z) * l.z;
-        const double lm = (p.x - rho.x) * l.x + (p.y - rho.y) * l.y + (p.z - rho.z) * l.z;
-        const double R02 = P0 * P0 + d * d;
-        const double Rp = sqrt(R02 + lp * lp), Rm = sqrt(R02 + lm * lm);
-        double f;
-        if (R02 < 1e-30 * (lp * lp + lm * lm)) {
-            f = 0.0;   // point on the edge line: the terms vanish
-        } else {
-            // f = log((Rp + lp)/(Rm + lm)); R + l = R02/(R - l) where l < 0 avoids the cancellation
-            const double np_ = lp >= 0.0 ? Rp + lp : R02 / (Rp - lp);
-            const double nm_ = lm >= 0.0 ? Rm + lm : R02 / (Rm - lm);
-            f = log(np_ / nm_);
-        }
-        double beta = 0.0;
-        if (ad > 0.0) beta = atan(P0 * lp / (R02 + ad * Rp)) - atan(P0 * lm / (R02 + ad * Rm));
-        s0 += P0 * f - ad * beta;
-        const double t = 0.5 * (R02 * f + lp * Rp - lm * Rm);
-        vx += u.x * t; vy += u.y * t; vz += u.z * t;
-    }
-    I0 = s0;
-    J = make_double3(vx - d * n.x * s0, vy - d * n.y * s0, vz - d * n.z * s0);
-}
-
 // (exp(-jkR) - 1)/(4 pi R) without cancellation; -jk/(4 pi) at R = 0
 __device__ __forceinline__ void smooth_green(double kr, double ki, double R, double &gr, double &gi) {
     if (R == 0.0) {
@@ -1167,6 +1122,10 @@ efie_status efie_geom_upload(efie_ctx *ctx, const efie_mesh *mesh, const efie_pr
                         list.push_back(make_int2(t1, t2));
                     }
         }
+        // ordered by (t2, t1) like the near list
+        std::sort(list.begin(), list.end(), [](const int2 &a, const int2 &b) {
+            return a.y != b.y ? a.y < b.y : a.x < b.x;
+        });
         g.symmetric = true;
         g.n_adj = (int)list.size();
         g.n_near = 0;
@@ -1198,22 +1157,30 @@ efie_status efie_geom_upload(efie_ctx *ctx, const efie_mesh *mesh, const efie_pr
         g.n_reg_tiles = (int)tl.size();
         EFIE_TRY(up(g.reg_tiles, tl.data(), sizeof(int2) * tl.size()));
     }
-    // component planes of npairs (9 edge combinations or the 8 moments) for up
-    // to four frequencies assembled together, within a quarter of free memory
-    const size_t per = sizeof(double2) * (g.combo ? 9 : 8) * g.npairs;
-    size_t freeb = 0, totalb = 0;
-    g.mf = 1;
-    if ((g.Nq == 3 || g.Nq == 7) && cudaMemGetInfo(&freeb, &totalb) == cudaSuccess)
-        for (int f = 4; f >= 2; f--)
-            if (f * per <= freeb / 4) {
-                g.mf = f;
-                break;
-            }
-    EFIE_TRY(g.moments.reserve(per * g.mf));
     return EFIE_OK;
 }
 
 namespace {
+
+// The pair values' buffer, reserved by the first assembly that needs them (a
+// sweep on the series assembly never does): component planes of npairs (9
+// edge combinations or the 8 moments) for up to four frequencies assembled
+// together, within a quarter of free memory or the buffer at hand.
+efie_status pair_values(GeomDev &g) {
+    if (g.mf > 0) return EFIE_OK;
+    const size_t per = sizeof(double2) * (g.combo ? 9 : 8) * g.npairs;
+    size_t freeb = 0, totalb = 0;
+    int mf = 1;
+    if ((g.Nq == 3 || g.Nq == 7) && cudaMemGetInfo(&freeb, &totalb) == cudaSuccess)
+        for (int f = 4; f >= 2; f--)
+            if (f * per <= std::max(freeb / 4, g.moments.bytes)) {
+                mf = f;
+                break;
+            }
+    EFIE_TRY(g.moments.reserve(per * mf));
+    g.mf = mf;
+    return EFIE_OK;
+}
 
 // the pair-value store of frequency slot j of the geometry's moment buffer
 MomStore mom_store(const GeomDev &g, const Physics &ph, int j) {
@@ -1289,6 +1256,7 @@ efie_status efie_assemble_finish(efie_ctx *ctx, GeomDev &g, const Physics &ph, i
 efie_status efie_assemble_device(efie_ctx *ctx, GeomDev &g, const Physics &ph, void *Z, float *pr, int ld) {
     cudaStream_t s = ctx->stream;
     KernelLog &log = ctx->log;
+    EFIE_TRY(pair_values(g));
     const int Nt = g.Nt;
     const MomStore mom = mom_store(g, ph, 0);
     dim3 grid((Nt + 31) / 32, (Nt + 7) / 8);
@@ -1315,6 +1283,7 @@ efie_status efie_assemble_device(efie_ctx *ctx, GeomDev &g, const Physics &ph, v
 efie_status efie_assemble_batch(efie_ctx *ctx, GeomDev &g, const Physics *ph, int nf, void *const *Z,
                                 const PlanesOut *po) {
     if (po && !g.symmetric) return efie_fail(EFIE_ERR_ARGS, "complex64 planes need the symmetric gather");
+    EFIE_TRY(pair_values(g));
     auto planes = [&](int f) { return po ? po->p + po->pstride * f : nullptr; };
     const int ld = po ? po->ld : 0;
     int f0 = 0;

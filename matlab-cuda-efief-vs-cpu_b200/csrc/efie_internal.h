@@ -172,12 +172,21 @@ struct GeomDev {
     DevBuf moments;           // double2[9 or 8][npairs]: component-major pair values (assemble.cu)
     size_t npairs = 0;
     bool combo = false;       // edge-combination form (9 values per pair) in use
-    int mf = 1;               // frequencies whose pair values fit the moment buffer together
+    int mf = 0;               // frequencies whose pair values fit the moment buffer together (0: none reserved yet)
     DevBuf tri_d;             // double4[3*Nt] free-vertex vectors per triangle slot
     DevBuf edge_tl;           // int32[2*Ne] 4 t + slot per RWG side (-1 = none)
     DevBuf edge_c;            // double[2*Ne] RWG coefficient c per side
     DevBuf reg_tiles;         // int2[n_reg_tiles] (t1 block, t2 block) of the symmetric regular-pair launches
     int n_reg_tiles = 0;
+    // series assembly (series.cu): RWG centres, half-width of R - R0 (0 until
+    // the first sweep measures it), coefficients of a batch, special pairs'
+    // moments, and the moments of the entries in `moments` (ser_cap of the
+    // ser_tiles tiles at a time; ser_done: all of this sweep's are there)
+    DevBuf ser_ctr, ser_coef, ser_sp;
+    double ser_delta = 0.0;
+    int ser_n = 0;            // terms of the current sweep
+    size_t ser_cap = 0, ser_tiles = 0;
+    bool ser_done = false;
 };
 
 // Per-frequency physics: k = w sqrt(mu eps) (principal branch), alpha = j w mu,
@@ -217,6 +226,14 @@ struct PlanesOut {
 // regular-pair evaluation), and into the planes of slots 0 .. nf-1 when po is set
 efie_status efie_assemble_batch(efie_ctx *ctx, GeomDev &g, const Physics *ph, int nf, void *const *Z,
                                 const PlanesOut *po = nullptr);
+// series.cu: a sweep's assembly from frequency-independent moments.  begin
+// (once per sweep; kabs, kimag: the largest |k| and |Im k|) tells whether the
+// series serves the sweep; assemble then writes nf frequencies into the slots
+// at Z (Z's upper triangle and its 128 x 128 diagonal blocks), and into the
+// planes' lower triangle when po is set.
+efie_status efie_series_begin(efie_ctx *ctx, GeomDev &g, double kabs, double kimag, bool *use);
+efie_status efie_series_assemble(efie_ctx *ctx, GeomDev &g, const Physics *ph, int nf, void *Z, size_t zstride,
+                                 const PlanesOut *po);
 efie_status efie_assemble_centroid_device(efie_ctx *ctx, const efie_mesh *mesh, double selfAlpha,
                                           const Physics &ph, void *Z, DevBuf &scratch);
 #endif
