@@ -192,8 +192,9 @@ typedef struct efie_sweep_opts {
                                 factors of the nearest frequency of that batch, which
                                 stay in the plan's slots, and the automatic batch
                                 size gives a sweep at least g batches.  1: every
-                                frequency is factored.  0 (default): automatic,
-                                g ~ Ne / 1200 within [2, 8] */
+                                frequency is factored.  0 (default): automatic, a
+                                first batch of 3 to 24 frequencies (48000 / Ne, at
+                                most what the band needs) is factored for all */
 } efie_sweep_opts;
 
 /* Fill `o` with the defaults listed above. */
@@ -418,6 +419,13 @@ void efie_debug_disable_warm_start(int disable);
  * left alone).  No counterpart in the reference. */
 efie_status efie_debug_plan_series(efie_plan *plan, const double *freqs, int32_t nf, int32_t tiles, int32_t *terms,
                                    efie_c128 *Z);
+
+/* The initial guess of a sweep's refinement on its own: the combination x of
+ * the k (at most 23) vectors xs [k][N] with the smallest || b - Z x ||, for a
+ * symmetric Z [N x N] of which the upper triangle and the 128 x 128 diagonal
+ * blocks are read.  No counterpart in the reference. */
+efie_status efie_debug_snapshot_guess(efie_ctx *ctx, int32_t N, int32_t k, const efie_c128 *Z, const efie_c128 *xs,
+                                      const efie_c128 *b, efie_c128 *x);
 
 /* ---------------------------------------------------------------------- */
 /* Centroid assembly without device allocation                             */

@@ -298,7 +298,7 @@ def sweep_opts(solver="mixed", port_model="gauss", scheme="ref", refine_tol=1e-1
     share_factors: g >= 2 factors only the first of each group of g
     coarse-to-fine batches, the others refine with the factors of their
     nearest neighbours in it; 1: every frequency is factored; 0: automatic
-    (g ~ Ne / 1200 within [2, 8])."""
+    (one batch of 3 to 24 frequencies is factored for the sweep)."""
     o = nat.EfieSweepOpts()
     nat.lib().efie_sweep_opts_default(C.byref(o))
     o.solver = {"fp64": nat.SOLVER_FP64, "mixed": nat.SOLVER_MIXED}[solver]

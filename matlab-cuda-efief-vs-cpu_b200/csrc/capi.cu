@@ -402,6 +402,8 @@ struct efie_plan {
     int Ne = 0;
     int B = 1;                   // frequencies per batch
     int share_group = 1;         // batches per factored batch (1: every frequency factored)
+    bool auto_share = false;     // automatic sharing (choose_anchors)
+    double extent = 0.0;         // diagonal of the vertices' bounding box
     double mu = 0, V0 = 0, Z0 = 0;
     efie_c128 eps{0, 0};
     int pe = 0, ge = 0;
@@ -523,8 +525,23 @@ int choose_share_group(int N, int requested) {
     return std::max(2, std::min(8, (int)std::lround(N / 1200.0)));
 }
 
+// Automatic sharing: a sweep factors some frequencies (anchors); the others
+// refine with the nearest one's factors, from a combination of solved currents
+// that leaves most of them no GMRES step to do (snapshot.cu).
+//
+// Solved frequencies that carry a sweep's currents to about 1e-10: measured 13
+// for a phase of 1.8 rad across the structure over the band (Ne 1074, 2-3 GHz)
+// and about 20 for 3.3 rad (Ne 2382, f0 +- 20 %).
+int snapshots_wanted(double phase) { return (int)std::min(24.0, std::ceil(8.0 + 3.5 * phase)); }
+// Of these, factored: all where the factorization is latency bound (1.8 ms for
+// one frequency of Ne 1074, 2.0 for sixteen), few where its O(N^3) counts (Ne
+// 6968: 2.2 ms each, Ne 19936: 30 ms each, against 0.16 and 1.5 ms for a GMRES
+// step with a neighbour's factors).
+int choose_anchors(int N) { return std::max(3, std::min(24, (int)std::lround(48000.0 / N))); }
+
 // group: batches per factored batch with shared factors (> 1): a sweep of nf
-// frequencies then has at least that many batches
+// frequencies then has at least that many batches; 0: automatic sharing, the
+// batch holds the factored frequencies and an even share of the others.
 int choose_batch(int N, int requested, int solver, int nf, int group = 1) {
     if (solver == EFIE_SOLVER_FP64) return 1;
     if (requested > 0) return std::min(requested, EFIE_MAX_BATCH);
@@ -536,7 +553,15 @@ int choose_batch(int N, int requested, int solver, int nf, int group = 1) {
     const double per = 26.0 * (double)N * N + 1e6;
     int B = (int)std::floor(0.45 * (double)freeb / per);
     B = std::max(1, std::min(B, N >= 4096 ? EFIE_MAX_BATCH : 32));
-    if (nf > 0) {
+    if (nf > 0 && group == 0) {
+        const int na = choose_anchors(N), rest = nf - na;
+        if (rest <= 0) return std::min(B, nf);
+        // small problems: as few batches as fit (each costs its launches);
+        // larger ones up to four, which bounds the memory of long sweeps
+        int nbat = (rest + B - 1) / B;
+        if (N >= 4096) nbat = std::max(nbat, std::min(4, (rest + 7) / 8));
+        B = std::min(B, std::max(na, (rest + nbat - 1) / nbat));
+    } else if (nf > 0) {
         const int nbat = std::max((nf + B - 1) / B, std::min(std::max(group, 1), nf));
         B = (nf + nbat - 1) / nbat;
     }
@@ -587,7 +612,15 @@ efie_status plan_common(efie_plan *p, const efie_mesh *mesh, double mu, efie_c12
     p->share_group = p->opts.solver == EFIE_SOLVER_MIXED && p->opts.refine_method == EFIE_REFINE_GMRES
                          ? choose_share_group(N, p->opts.share_factors)
                          : 1;
-    p->B = choose_batch(N, p->opts.batch, p->opts.solver, p->opts.nfreq_hint, p->share_group);
+    double box = 0.0;
+    for (int k = 0; k < 3; k++) {
+        const double *v = mesh->V + (size_t)k * mesh->Nv;
+        const auto mm = std::minmax_element(v, v + mesh->Nv);
+        box += (*mm.second - *mm.first) * (*mm.second - *mm.first);
+    }
+    p->extent = std::sqrt(box);
+    p->auto_share = p->share_group > 1 && p->opts.share_factors <= 0;
+    p->B = choose_batch(N, p->opts.batch, p->opts.solver, p->opts.nfreq_hint, p->auto_share ? 0 : p->share_group);
     EFIE_TRY(p->Z.reserve(sizeof(efie_c128) * (size_t)N * N * p->B));
     EFIE_TRY(p->b.reserve(sizeof(efie_c128) * N));
     EFIE_TRY(p->x.reserve(sizeof(efie_c128) * (size_t)N * p->B));
@@ -757,6 +790,28 @@ extern "C" efie_status efie_debug_plan_series(efie_plan *p, const double *freqs,
     return EFIE_OK;
 }
 
+// The nearest solved frequencies (up to `most`) of each frequency of a batch;
+// false with fewer than three solved, where interpolation does as well.
+static bool snapshot_nodes(const int *pos, int nb, const std::vector<double> &fs, const std::vector<char> &solved,
+                           int most, SnapSpec &g) {
+    std::vector<int> s;
+    for (int q = 0; q < (int)fs.size(); q++)
+        if (solved[q]) s.push_back(q);
+    if (s.size() < 3) return false;
+    const int k = std::min<int>(most, (int)s.size());
+    g = SnapSpec{};
+    for (int f = 0; f < nb; f++) {
+        const double x = fs[pos[f]];
+        std::partial_sort(s.begin(), s.begin() + k, s.end(), [&](int a, int b) {
+            const double da = std::abs(fs[a] - x), db = std::abs(fs[b] - x);
+            return da != db ? da < db : a < b;
+        });
+        g.k[f] = k;
+        for (int t = 0; t < k; t++) g.pos[f][t] = s[t];
+    }
+    return true;
+}
+
 static bool g_warm_start_disabled = false;
 extern "C" void efie_debug_disable_warm_start(int disable) { g_warm_start_disabled = disable != 0; }
 
@@ -789,9 +844,24 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
     // q = r_b (mod nbat), residues in van der Corput order, so every later
     // frequency starts its refinement from the interpolation of its solved
     // neighbours instead of from zero.
-    const int nbat = (Nf + B - 1) / B;
-    const bool warm = mixed && !p->centroid && nbat > 1 && p->opts.refine_method == EFIE_REFINE_GMRES &&
-                      !g_warm_start_disabled;
+    // With automatic sharing the first batch holds the factored frequencies
+    // (anchors), spread over the band, and the others follow farthest from the
+    // solved ones first.
+    const bool refines = mixed && !p->centroid && p->opts.refine_method == EFIE_REFINE_GMRES &&
+                         !g_warm_start_disabled;
+    double kmin = 1e300, kmax = 0.0;
+    for (int fi = 0; fi < Nf; fi++) {
+        const double k = efie_physics(freqs[fi], p->mu, p->eps).kr;
+        kmin = std::min(kmin, k);
+        kmax = std::max(kmax, k);
+    }
+    const int wanted = snapshots_wanted(Nf > 0 ? (kmax - kmin) * p->extent : 0.0);
+    const int na = std::min({Nf, wanted, choose_anchors(N)});
+    const bool anchored = refines && p->auto_share && p->sw.zsym && p->sw.sym_lu && na <= B;
+    const int lvl1 = anchored && Nf - na > 2 * (wanted - na) ? std::min(B, wanted - na) : 0;
+    const int tail = anchored ? (Nf - na - lvl1 + B - 1) / B : 0;   // batches of the remaining frequencies
+    const int nbat = anchored ? 1 + (lvl1 > 0) + tail : (Nf + B - 1) / B;
+    const bool warm = refines && nbat > 1;
     std::vector<int> ord(Nf), bstart(nbat + 1, 0), posq(Nf);   // processing index -> original, sorted position
     std::vector<double> fsorted(Nf);
     std::vector<char> solved(Nf, 0);
@@ -800,19 +870,76 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
         for (int i = 0; i < Nf; i++) srt[i] = i;
         if (warm) std::stable_sort(srt.begin(), srt.end(), [&](int a, int b) { return freqs[a] < freqs[b]; });
         for (int i = 0; i < Nf; i++) fsorted[i] = freqs[srt[i]];
-        int n = 0, P = 1, bits = 0;
-        while (P < nbat) P <<= 1, bits++;
-        for (int i = 0, b = 0; i < (warm ? P : nbat); i++) {
-            if (warm) {
+        // residues 0 .. count-1 in van der Corput order
+        auto residues = [](int count) {
+            std::vector<int> v;
+            int P = 1, bits = 0;
+            while (P < count) P <<= 1, bits++;
+            for (int i = 0; i < P; i++) {
                 int r = 0;
                 for (int t = 0; t < bits; t++) r |= ((i >> t) & 1) << (bits - 1 - t);
-                if (r >= nbat) continue;
-                for (int q = r; q < Nf; q += nbat) posq[n] = q, ord[n++] = srt[q];
-            } else {
-                const int nb = Nf / nbat + (b < Nf % nbat ? 1 : 0);
-                for (int f = 0; f < nb; f++) posq[n] = n, ord[n] = srt[n], n++;
+                if (r < count) v.push_back(r);
+            }
+            return v;
+        };
+        int n = 0, b = 0;
+        auto put = [&](int q) { posq[n] = q, ord[n++] = srt[q]; };
+        if (anchored) {
+            std::vector<char> taken(Nf, 0);
+            std::vector<int> aq(na);
+            for (int i = 0; i < na; i++) {
+                if (na < wanted || na < 3) {   // the middles of equal parts: what a neighbour shares lies near
+                    aq[i] = (int)(((2 * (int64_t)i + 1) * Nf) / (2 * (int64_t)na));
+                } else {                       // all the snapshots there will be: Chebyshev points hold the ends
+                    const double t = 0.5 * (1.0 - std::cos(3.14159265358979324 * i / (na - 1)));
+                    const double f = fsorted[0] + t * (fsorted[Nf - 1] - fsorted[0]);
+                    const int q = (int)(std::lower_bound(fsorted.begin(), fsorted.end(), f) - fsorted.begin());
+                    aq[i] = q >= Nf ? Nf - 1 : q > 0 && f - fsorted[q - 1] < fsorted[q] - f ? q - 1 : q;
+                }
+                if (i) aq[i] = std::max(aq[i], aq[i - 1] + 1);
+            }
+            for (int i = na - 1; i >= 0; i--) aq[i] = std::min(aq[i], i + 1 < na ? aq[i + 1] - 1 : Nf - 1);
+            for (int q : aq) {
+                taken[q] = 1;
+                put(q);
             }
             bstart[++b] = n;
+            if (lvl1 > 0) {
+                // each the farthest in frequency from every one taken so far
+                std::vector<double> dist(Nf, 1e300);
+                for (int q = 0; q < Nf; q++)
+                    for (int i = 0; i < na; i++) dist[q] = std::min(dist[q], std::abs(fsorted[q] - fsorted[posq[i]]));
+                std::vector<int> more;
+                for (int i = 0; i < lvl1; i++) {
+                    int best = -1;
+                    for (int q = 0; q < Nf; q++)
+                        if (!taken[q] && (best < 0 || dist[q] > dist[best])) best = q;
+                    taken[best] = 1;
+                    more.push_back(best);
+                    for (int q = 0; q < Nf; q++) dist[q] = std::min(dist[q], std::abs(fsorted[q] - fsorted[best]));
+                }
+                std::sort(more.begin(), more.end());
+                for (int q : more) put(q);
+                bstart[++b] = n;
+            }
+            std::vector<int> rest;
+            for (int q = 0; q < Nf; q++)
+                if (!taken[q]) rest.push_back(q);
+            for (int r : residues(tail)) {
+                for (size_t i = r; i < rest.size(); i += tail) put(rest[i]);
+                bstart[++b] = n;
+            }
+        } else if (warm) {
+            for (int r : residues(nbat)) {
+                for (int q = r; q < Nf; q += nbat) put(q);
+                bstart[++b] = n;
+            }
+        } else {
+            for (int i = 0; i < nbat; i++) {
+                const int nb = Nf / nbat + (b < Nf % nbat ? 1 : 0);
+                for (int f = 0; f < nb; f++) put(n);
+                bstart[++b] = n;
+            }
         }
     }
     if (warm) EFIE_TRY(p->xall.reserve(sizeof(efie_c128) * (size_t)N * Nf));
@@ -825,7 +952,7 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
     // the same residual target in a few more steps; a frequency that does
     // not gets the retry below, with its own factors -- which converts Z to
     // planes in every slot, so the rest of the group then factors itself.
-    const int group = p->share_group;   // batches per factored batch
+    const int group = anchored ? nbat : p->share_group;   // batches per factored batch
     const bool share = mixed && warm && group > 1 && p->sw.zsym && p->sw.sym_lu &&
                        p->opts.refine_method == EFIE_REFINE_GMRES;
     bool prev_factored = false;      // the slots hold the factors of the group's first batch
@@ -875,9 +1002,9 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
                 for (int f = 0; f < p->B; f++) fsrc_host[f] = f;
                 for (int f = 0; f < nb; f++) {
                     int best = 0;
+                    const double fq = fsorted[posq[f0 + f]];
                     for (int s2 = 1; s2 < np_; s2++)
-                        if (std::abs(posq[p0 + s2] - posq[f0 + f]) < std::abs(posq[p0 + best] - posq[f0 + f]))
-                            best = s2;
+                        if (std::abs(fsorted[posq[p0 + s2]] - fq) < std::abs(fsorted[posq[p0 + best]] - fq)) best = s2;
                     fsrc_host[f] = best;
                 }
                 rc = set_fsrc(false);
@@ -891,7 +1018,11 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
             if (!shared && bi % group == 0) prev_factored = true;
             RefineResult rr;
             const bool guess = warm && bi > 0;
-            if (guess) {
+            SnapSpec sp;
+            if (guess && share && snapshot_nodes(posq.data() + f0, nb, fsorted, solved, wanted > 15 ? EFIE_SNAP_MAX : 15, sp)) {
+                rc = efie_snapshot_guess(ctx, p->sw, p->Z.p, NN, p->xall.p, p->b.p, nb, sp, p->x.p);
+                if (rc != EFIE_OK) break;
+            } else if (guess) {
                 GuessSpec g;
                 for (int f = 0; f < nb; f++) guess_weights(posq[f0 + f], fsorted, solved, g, f);
                 rc = efie_interp_guess(ctx, N, nb, p->x.p, p->xall.p, g);

@@ -24,7 +24,7 @@
 //
 // Every kernel carries the frequency in its grid and returns at once for a
 // frequency whose cycle has stopped; the host polls the stop flags after
-// every step from the third on.  Per-frequency state lives in GmState (device memory).
+// every step (without an initial guess, from the third on).  Per-frequency state lives in GmState (device memory).
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -607,17 +607,17 @@ efie_status efie_mixed_gmres(efie_ctx *ctx, SolveWork &w, const void *Z, size_t 
     const double zbytes = 16.0 * (double)N * N, lubytes = 8.0 * (double)N * N;
     const double tol_inner = 0.5 * tol;
     const int *ctl_skip0 = reinterpret_cast<const int *>(ctl + 32);   // ctl skip flag of slot f: [16 f]
-    auto residual = [&]() -> efie_status {
-        if (!w.zsym) return efie_true_residual(ctx, w, Z, zstride, x, b, tol, V, nact);
+    auto residual = [&](double done) -> efie_status {   // done: the norm that counts as solved
+        if (!w.zsym) return efie_true_residual(ctx, w, Z, zstride, x, b, done, V, nact);
         size_t tk = log.begin(s);
         EFIE_TRY(symv(ctx, w, Z, zstride, static_cast<const double2 *>(x), wv, ctl_skip0, 16));
         log.end(EFIE_K_RESIDUAL, s, tk, 8.0 * (double)N * N * nact, 2);
-        return efie_residual_finish(ctx, w, wv, b, tol, V, nact);
+        return efie_residual_finish(ctx, w, wv, b, done, V, nact);
     };
     EFIE_TRY(efie_refine_init(ctx, w, x, bnorm, !x0_given));
     // r0 = b - Z x0, stored at V slot 0 too; for x0 = 0 without the product
     if (x0_given || !w.zsym) {
-        EFIE_TRY(residual());
+        EFIE_TRY(residual(tol_inner));   // a guess is held to what the cycles aim at
     } else {
         EFIE_CUDA(cudaMemsetAsync(wv, 0, sizeof(double2) * (size_t)N * B, s));
         EFIE_TRY(efie_residual_finish(ctx, w, wv, b, tol, V, nact));
@@ -625,10 +625,26 @@ efie_status efie_mixed_gmres(efie_ctx *ctx, SolveWork &w, const void *Z, size_t 
     std::vector<char> hctl(64 * (size_t)B);
     std::vector<int> hstop(B);
     int matvecs = 0;
+    bool all_conv = false, failed = false;
+    // ctl of the batch to the host after a true residual
+    auto read_ctl = [&](int &running) -> efie_status {
+        EFIE_CUDA(cudaMemcpyAsync(hctl.data(), ctl, 64 * (size_t)B, cudaMemcpyDeviceToHost, s));
+        EFIE_CUDA(cudaStreamSynchronize(s));
+        all_conv = true;
+        running = 0;
+        for (int f = 0; f < B; f++) {
+            if (!active_host[f]) continue;
+            const char *c = hctl.data() + 64 * f;
+            if (*reinterpret_cast<const int *>(c + 36)) failed = true;
+            if (!*reinterpret_cast<const int *>(c + 28)) all_conv = false, running++;
+        }
+        return EFIE_OK;
+    };
     // frequencies still iterating as of the last stop-flag poll: the work the
     // in-cycle launches count (a stopped frequency's CTAs return at once)
     int nrun = nact;
-    bool all_conv = false, failed = false;
+    // a guess may meet the target by itself
+    if (x0_given) EFIE_TRY(read_ctl(nrun));
     const dim3 vg(cdiv(N, 256), B), og(nch, B), mg(cdiv(N, 32), B);
     while (!all_conv && !failed && matvecs < max_iter) {
         size_t tok = log.begin(s);
@@ -664,7 +680,7 @@ efie_status efie_mixed_gmres(efie_ctx *ctx, SolveWork &w, const void *Z, size_t 
             EFIE_CUDA(cudaGetLastError());
             log.end(EFIE_K_OTHER, s, tok, 32.0 * (double)N * (j + 1) * 2 * nrun, 7);
             matvecs++;
-            if (j >= 2) {
+            if (j >= (x0_given ? 0 : 2)) {   // a guess may be a step from the target
                 // a poll costs one synchronisation (tens of us) against a step
                 // of the whole batch (milliseconds at large N)
                 bool all_stop = true;
@@ -690,17 +706,8 @@ efie_status efie_mixed_gmres(efie_ctx *ctx, SolveWork &w, const void *Z, size_t 
         EFIE_CUDA(cudaGetLastError());
         log.end(EFIE_K_OTHER, s, tok, 0.0, 3);
         // true residual; a restart begins from it
-        EFIE_TRY(residual());
-        EFIE_CUDA(cudaMemcpyAsync(hctl.data(), ctl, 64 * (size_t)B, cudaMemcpyDeviceToHost, s));
-        EFIE_CUDA(cudaStreamSynchronize(s));
-        all_conv = true;
-        nrun = 0;
-        for (int f = 0; f < B; f++) {
-            if (!active_host[f]) continue;
-            const char *c = hctl.data() + 64 * f;
-            if (*reinterpret_cast<const int *>(c + 36)) failed = true;
-            if (!*reinterpret_cast<const int *>(c + 28)) all_conv = false, nrun++;
-        }
+        EFIE_TRY(residual(tol));
+        EFIE_TRY(read_ctl(nrun));
     }
     res->iters = matvecs;
     for (int f = 0; f < B; f++) {

@@ -710,15 +710,15 @@ efie_status efie_series_begin(efie_ctx *ctx, GeomDev &g, double kabs, double kim
             break;
         }
     if (!N) return EFIE_OK;
-    // the moments share the buffer of the pair values, within their quarter of
-    // free memory; what does not fit is made a part at a time, for every batch
+    // the moments share the buffer of the pair values, within a third of free
+    // memory; what does not fit is made a part at a time, for every batch
     const size_t nb = (g.Ne + TE - 1) / TE, tiles = nb * (nb + 1) / 2;
     const size_t per = sizeof(double) * 2 * N * TE * TE, old = g.moments.bytes;
     if (tiles > (size_t)1 << 30) return EFIE_OK;
     if (old < tiles * per) {
         size_t freeb = 0, total = 0;
         if (cudaMemGetInfo(&freeb, &total) != cudaSuccess) return EFIE_OK;
-        const size_t most = (freeb + efie_pool_cached(ctx->device) + old) / 4 / per;
+        const size_t most = (freeb + efie_pool_cached(ctx->device) + old) / 3 / per;
         const size_t want = std::min(tiles, most) * per;
         if (want > old) {
             EFIE_CUDA(cudaStreamSynchronize(s));   // an earlier assembly may still read it

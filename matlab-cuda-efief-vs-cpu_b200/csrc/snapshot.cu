@@ -1,0 +1,451 @@
+// Initial guesses of a batch from the solutions of the sweep's solved
+// frequencies (snapshots).
+//
+// The currents of a sweep move in a space of few dimensions, so the combination
+// of the nearest snapshots x_j that minimises || b - Z(f) sum c_j x_j || starts
+// the refinement of frequency f far below any fixed interpolation weights:
+// measured (Ne 1074, 2-3 GHz, snapshots 60 MHz apart solved to 1e-10), four
+// snapshots leave 3e-5 of ||b||, eight 4e-10 and twelve 1e-11, where the
+// quadratic through three leaves 5e-3.  From twelve on most frequencies meet
+// the residual target before their first GMRES step.
+//
+//   W = Z(f) [x_1 .. x_k]   one product kernel for all vectors (k_symv_multi)
+//   [W b] = Q R             tall-skinny Householder QR, two launches
+//   c = R^-1 Q^H b          (nearly dependent columns get c = 0), x0 = sum c_j x_j
+// The Householder form keeps the digits that the snapshots' near dependence
+// would cost the normal equations; the refinement then starts from the true
+// residual of x0, so the guess never decides what counts as solved.
+#include <algorithm>
+#include <vector>
+
+#include "efie_internal.h"
+#include "solve.h"
+#include "tma.h"
+
+namespace {
+
+using namespace efie_tma;
+
+constexpr int KMAX = EFIE_SNAP_MAX;   // snapshots per frequency
+// columns of [W b] in the QR: 16 (up to 15 snapshots) or 24
+static_assert(KMAX == 23, "the wider QR holds 24 columns");
+
+// ---------------------------------------------------------------------------
+// W_f = Z_f X_f for up to K vectors, Z symmetric (upper triangle and full
+// 128 x 128 diagonal blocks stored).  An item is a block of 128 rows I of one
+// frequency: its y_I stays in registers over all blocks J, from tile (I, J)
+// as stored for J >= I and from the stored tile (J, I) transposed below, so
+// there are no partial vectors and no sums across tiles; Z is read twice
+// (once from L2 where the two readers meet), which the FP64 pipe hides: a
+// 64 KB chunk costs 64 K multiply-adds per lane, as long as HBM takes for it
+// at K = 12.  Chunks are 32 of the contraction's entries, through a ring of
+// three stages: boxes of 8 rows (128 bytes) in the 128-byte swizzle, so that
+// eight lanes on eight rows of one column (as stored) and on eight columns of
+// one row (transposed) both touch eight different 16-byte banks.  Lane
+// (l & 7, l >> 3) of warp w owns y_I[16 w + (l & 7)] and y_I[16 w + 8 + (l & 7)]
+// over every fourth entry; the X slices of the chunk come with it in the stage.
+// ---------------------------------------------------------------------------
+constexpr int MB = 128;                             // rows per item
+constexpr int MC = 32;                              // contraction entries per chunk
+constexpr int MR = 3;                               // stages
+constexpr uint32_t MZ = MB * MC * sizeof(double2);  // 64 KB of Z per chunk
+constexpr uint32_t MX = MC * sizeof(double2);       // one vector's slice
+
+template <int K>
+constexpr size_t multi_smem() {
+    return MR * (size_t)(MZ + K * MX) + 1024 + 64;
+}
+
+struct SnapIdx {
+    const int *k;     // [nf] snapshots of each frequency
+    const int *pos;   // [nf][KMAX] their rows of xall, nearest first
+};   // a launch takes vectors v0 .. v0 + K - 1 into those columns of W [nf][ldw][N]
+
+template <int K>
+__global__ void __launch_bounds__(256, 1) k_symv_multi(const __grid_constant__ CUtensorMap dmap,
+                                                       const __grid_constant__ CUtensorMap tmap, int N, int nb, int nf,
+                                                       const double2 *__restrict__ xall, const SnapIdx S,
+                                                       double2 *__restrict__ W, int v0, int ldw, char *ctl) {
+    extern __shared__ unsigned char dsm[];
+    __shared__ int fail;
+    constexpr uint32_t STAGE = MZ + K * MX;
+    unsigned char *ring = dsm + (((smem_u32(dsm) + 1023u) & ~1023u) - smem_u32(dsm));
+    uint64_t *full = reinterpret_cast<uint64_t *>(ring + MR * STAGE);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int G = gridDim.x, items = nb * nf;
+    // slices past row N are not copied: what a stage holds there must be finite
+    for (int i = tid; i < MR * K * MC; i += 256)
+        reinterpret_cast<double2 *>(ring + (i / (K * MC)) * STAGE + MZ)[i % (K * MC)] = make_double2(0.0, 0.0);
+    int p_it = blockIdx.x, p_q = 0, issued = 0;   // producer (thread 0): chunk p_q of item p_it is next
+    auto produce = [&]() {
+        if (p_it >= items) return;
+        const int f = p_it / nb, I = p_it - f * nb, J = p_q >> 2, n0 = J * MB + (p_q & 3) * MC;
+        unsigned char *st = ring + (issued % MR) * STAGE;
+        uint64_t *bar = full + issued % MR;
+        const int kf = min(K, max(0, S.k[f] - v0)), cnt = max(0, min(MC, N - n0));
+        mbar_expect_tx(bar, MZ + (uint32_t)(kf * cnt) * sizeof(double2));
+        if (J >= I)
+            for (int b = 0; b < MB / 8; b++) tma_load_3d(&dmap, st + b * 4096, 2 * (I * MB + 8 * b), n0, f, bar);
+        else
+            for (int b = 0; b < MC / 8; b++) tma_load_3d(&tmap, st + b * 16384, 2 * (n0 + 8 * b), I * MB, f, bar);
+        if (cnt > 0)
+            for (int v = 0; v < kf; v++)
+                bulk_g2s(st + MZ + v * MX, xall + (size_t)N * S.pos[f * KMAX + v0 + v] + n0,
+                         (uint32_t)cnt * sizeof(double2), bar);
+        issued++;
+        if (++p_q == 4 * nb) p_q = 0, p_it += G;
+    };
+    if (tid == 0) {
+        for (int s = 0; s < MR; s++) mbar_init(full + s, 1);
+        mbar_init_fence();
+        fail = 0;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the zeros before the copies
+    __syncthreads();
+    if (tid == 0)
+        for (int s = 0; s < MR; s++) produce();
+    const int li = lane & 7, g = lane >> 3;
+    int cc = 0;
+    for (int it = blockIdx.x; it < items; it += G) {
+        const int f = it / nb, I = it - f * nb;
+        double2 acc[2][K];
+#pragma unroll
+        for (int v = 0; v < K; v++) acc[0][v] = acc[1][v] = make_double2(0.0, 0.0);
+#pragma unroll 1
+        for (int q = 0; q < 4 * nb; q++) {
+            if (!mbar_wait_bounded(full + cc % MR, (uint32_t)(cc / MR) & 1u)) fail = 1;
+            const unsigned char *st = ring + (cc % MR) * STAGE;
+            if (!fail) {
+                const double2 *X = reinterpret_cast<const double2 *>(st + MZ);
+                const bool direct = (q >> 2) >= I;   // block-uniform
+#pragma unroll 1
+                for (int c8 = 0; c8 < MC / 4; c8++) {
+                    const int c = 4 * c8 + g;
+                    const unsigned char *p0, *p1;
+                    if (direct) {
+                        p0 = st + (2 * warp) * 4096 + c * 128 + ((li ^ (c & 7)) << 4);
+                        p1 = p0 + 4096;
+                    } else {
+                        p0 = st + (c >> 3) * 16384 + (16 * warp + li) * 128 + (((c & 7) ^ li) << 4);
+                        p1 = p0 + 8 * 128;
+                    }
+                    const double2 a0 = *reinterpret_cast<const double2 *>(p0);
+                    const double2 a1 = *reinterpret_cast<const double2 *>(p1);
+#pragma unroll
+                    for (int v = 0; v < K; v++) {
+                        const double2 x = X[v * MC + c];
+                        acc[0][v].x = fma(a0.x, x.x, fma(-a0.y, x.y, acc[0][v].x));
+                        acc[0][v].y = fma(a0.x, x.y, fma(a0.y, x.x, acc[0][v].y));
+                        acc[1][v].x = fma(a1.x, x.x, fma(-a1.y, x.y, acc[1][v].x));
+                        acc[1][v].y = fma(a1.x, x.y, fma(a1.y, x.x, acc[1][v].y));
+                    }
+                }
+            }
+            __syncthreads();   // every warp is done with the stage
+            if (fail) {
+                // a chunk never arrived: every frequency of the launch falls back
+                if (tid < nf) atomicExch(reinterpret_cast<int *>(ctl + 64 * tid + 36), 3);
+                if (tid == 0)
+                    for (int k = cc + 1; k < issued; k++)
+                        if (!mbar_wait_bounded(full + k % MR, (uint32_t)(k / MR) & 1u)) break;
+                return;
+            }
+            if (tid == 0) produce();
+            cc++;
+        }
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+#pragma unroll
+            for (int v = 0; v < K; v++) {
+                double2 s = acc[r][v];
+#pragma unroll
+                for (int o = 8; o <= 16; o <<= 1) {
+                    s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+                    s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+                }
+                const int m = I * MB + 16 * warp + 8 * r + li;
+                if (g == (v & 3) && m < N && v0 + v < ldw) W[((size_t)f * ldw + v0 + v) * N + m] = s;
+            }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Householder reduction of a block of 256 rows x QC complex columns, one row
+// per thread in registers: afterwards threads 0..QC-1 hold the rows of R.  Per
+// column one reduction gives x^H a_c of every column; with v = x - alpha e_j
+// (alpha opposite to the pivot), v^H a_c = x^H a_c - conj(alpha) a_jc.
+// ---------------------------------------------------------------------------
+template <int QC>
+struct QrSmem {
+    double part[8][2 * QC];
+    double sum[2 * QC];
+    double2 piv[QC];
+};
+
+// sums of n = 32 or 16 values over the warp: lane l is left with value l mod n
+// (each step hands over half of the values still held)
+template <int n>
+__device__ __forceinline__ double warp_sums(double (&d)[n], int lane) {
+    if (n == 16)
+#pragma unroll
+        for (int i = 0; i < n; i++) d[i] += __shfl_xor_sync(0xffffffffu, d[i], 16);
+#pragma unroll
+    for (int o = n / 2; o > 0; o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < n / 2; i++) {
+            if (i >= o) break;
+            const double keep = up ? d[i + o] : d[i], send = up ? d[i] : d[i + o];
+            d[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    return d[0];
+}
+
+// x^H a_c over the warp for the n / 2 columns from c0 on
+template <int n, int QC>
+__device__ __forceinline__ double column_dots(const double2 (&a)[QC], double2 x, int c0, bool on, int lane) {
+    double d[n];
+#pragma unroll
+    for (int c = 0; c < n / 2; c++) {
+        const double2 y = a[c0 + c];
+        d[2 * c] = on ? x.x * y.x + x.y * y.y : 0.0;
+        d[2 * c + 1] = on ? x.x * y.y - x.y * y.x : 0.0;
+    }
+    return warp_sums<n>(d, lane);
+}
+
+template <int QC>
+__device__ __forceinline__ void householder(double2 (&a)[QC], QrSmem<QC> &S) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+    for (int j = 0; j < QC - 1; j++) {
+        const bool on = tid >= j;
+        // columns before j are finished; their sums are not used
+        S.part[warp][lane] = column_dots<32>(a, a[j], 0, on, lane);
+        if (QC == 24) {
+            const double d = column_dots<16>(a, a[j], QC - 8, on, lane);
+            if (lane < 16) S.part[warp][2 * QC - 16 + lane] = d;
+        }
+        if (tid == j)
+#pragma unroll
+            for (int c = 0; c < QC; c++) S.piv[c] = a[c];
+        __syncthreads();
+        if (tid < 2 * QC) {
+            double s = 0.0;
+#pragma unroll
+            for (int w = 0; w < 8; w++) s += S.part[w][tid];
+            S.sum[tid] = s;
+        }
+        __syncthreads();
+        const double n2 = S.sum[2 * j];
+        if (n2 > 0.0) {   // uniform
+            const double nrm = sqrt(n2), ap = hypot(S.piv[j].x, S.piv[j].y);
+            const double2 u = ap > 0.0 ? make_double2(S.piv[j].x / ap, S.piv[j].y / ap) : make_double2(1.0, 0.0);
+            const double2 alpha = make_double2(-u.x * nrm, -u.y * nrm);
+            const double tau = 1.0 / (nrm * (nrm + ap));
+            const double2 v = tid == j ? make_double2(a[j].x - alpha.x, a[j].y - alpha.y) : a[j];
+            if (on) {
+#pragma unroll
+                for (int c = j + 1; c < QC; c++) {
+                    const double2 p = S.piv[c];
+                    const double wr = tau * (S.sum[2 * c] - (alpha.x * p.x + alpha.y * p.y));
+                    const double wi = tau * (S.sum[2 * c + 1] - (alpha.x * p.y - alpha.y * p.x));
+                    a[c].x -= v.x * wr - v.y * wi;
+                    a[c].y -= v.x * wi + v.y * wr;
+                }
+                a[j] = tid == j ? alpha : make_double2(0.0, 0.0);
+            }
+        }
+        __syncthreads();   // sum, piv and part are free for the next column
+    }
+}
+
+// R of each block of 256 rows of [W b]: R[f][block][QC][QC]
+template <int QC>
+__global__ void __launch_bounds__(256) k_tsqr_local(int N, int ldw, const int *__restrict__ kf,
+                                                    const double2 *__restrict__ W, const double2 *__restrict__ b,
+                                                    double2 *__restrict__ R) {
+    __shared__ QrSmem<QC> S;
+    const int f = blockIdx.y, n = blockIdx.x * 256 + threadIdx.x, k = kf[f];
+    double2 a[QC];
+#pragma unroll
+    for (int c = 0; c < QC - 1; c++)
+        a[c] = n < N && c < k ? W[((size_t)f * ldw + c) * N + n] : make_double2(0.0, 0.0);
+    a[QC - 1] = n < N ? b[n] : make_double2(0.0, 0.0);
+    householder<QC>(a, S);
+    if (threadIdx.x < QC) {
+        double2 *out = R + (((size_t)f * gridDim.x + blockIdx.x) * QC + threadIdx.x) * QC;
+#pragma unroll
+        for (int c = 0; c < QC; c++) out[c] = a[c];
+    }
+}
+
+// The blocks' R stacked below the result so far and reduced, as many as 256
+// rows hold at a time, then the coefficients coef[f][KMAX] by back
+// substitution; a column that depends on the ones before it to 1e-13 of its
+// norm gets none.
+template <int QC>
+__global__ void __launch_bounds__(256) k_tsqr_combine(int nblk, const int *__restrict__ kf,
+                                                      const double2 *__restrict__ R, double2 *__restrict__ coef) {
+    __shared__ QrSmem<QC> S;
+    __shared__ double2 T[QC][QC];
+    const int f = blockIdx.x, tid = threadIdx.x;
+    constexpr int PASS = 256 / QC - 1;
+    double2 a[QC];
+#pragma unroll
+    for (int c = 0; c < QC; c++) a[c] = make_double2(0.0, 0.0);
+    for (int b0 = 0; b0 < nblk; b0 += PASS) {
+        const int p = tid / QC - 1, blk = b0 + p, row = tid % QC;
+        if (tid >= QC) {
+            const bool in_range = p < PASS && blk < nblk;
+            const double2 *in = R + (((size_t)f * nblk + (in_range ? blk : 0)) * QC + row) * QC;
+#pragma unroll
+            for (int c = 0; c < QC; c++) a[c] = in_range ? in[c] : make_double2(0.0, 0.0);
+        }
+        householder<QC>(a, S);
+    }
+    if (tid < QC)
+#pragma unroll
+        for (int c = 0; c < QC; c++) T[tid][c] = a[c];
+    __syncthreads();
+    if (tid == 0) {
+        double2 x[QC - 1];
+        const int k = kf[f];
+        for (int j = QC - 2; j >= 0; j--) {
+            double2 s = T[j][QC - 1];
+            double col = 0.0;
+            for (int i = 0; i <= j; i++) col += T[i][j].x * T[i][j].x + T[i][j].y * T[i][j].y;
+            for (int i = j + 1; i < k; i++) {
+                s.x -= T[j][i].x * x[i].x - T[j][i].y * x[i].y;
+                s.y -= T[j][i].x * x[i].y + T[j][i].y * x[i].x;
+            }
+            const double2 d = T[j][j];
+            const double dn = d.x * d.x + d.y * d.y;
+            x[j] = j < k && dn > 1e-26 * col
+                       ? make_double2((s.x * d.x + s.y * d.y) / dn, (s.y * d.x - s.x * d.y) / dn)
+                       : make_double2(0.0, 0.0);
+            if (j < k) coef[f * KMAX + j] = x[j];
+        }
+    }
+}
+
+// x_f = sum_j c_j x_j
+__global__ void __launch_bounds__(256) k_snap_x(int N, const double2 *__restrict__ xall, const SnapIdx S,
+                                                const double2 *__restrict__ coef, double2 *__restrict__ x) {
+    const int f = blockIdx.y, n = blockIdx.x * 256 + threadIdx.x;
+    if (n >= N) return;
+    double2 s = make_double2(0.0, 0.0);
+    const int k = S.k[f];
+    for (int j = 0; j < k; j++) {
+        const double2 c = coef[f * KMAX + j], v = xall[(size_t)N * S.pos[f * KMAX + j] + n];
+        s.x += c.x * v.x - c.y * v.y;
+        s.y += c.x * v.y + c.y * v.x;
+    }
+    x[(size_t)N * f + n] = s;
+}
+
+// The two maps of Z (all slots) as doubles [B][N][2N]: boxes of 8 rows x 32
+// columns (tiles as stored) and 8 rows x 128 columns (tiles read transposed)
+efie_status multi_maps(int N, int B, const void *Z, size_t zstride, CUtensorMap *d, CUtensorMap *t) {
+    const cuuint64_t dims[3] = {2 * (cuuint64_t)N, (cuuint64_t)N, (cuuint64_t)B};
+    const cuuint64_t strides[2] = {sizeof(double2) * (cuuint64_t)N, sizeof(double2) * (cuuint64_t)zstride};
+    const cuuint32_t bd[3] = {16, MC, 1}, bt[3] = {16, MB, 1};
+    EFIE_TRY(efie_encode_tiled(d, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<void *>(Z), dims, strides, bd,
+                               CU_TENSOR_MAP_SWIZZLE_128B));
+    return efie_encode_tiled(t, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<void *>(Z), dims, strides, bt,
+                             CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+template <int K>
+efie_status launch_multi(efie_ctx *ctx, const CUtensorMap &d, const CUtensorMap &t, int N, int nf,
+                         const double2 *xall, const SnapIdx &S, double2 *W, int v0, int ldw, char *ctl) {
+    const int nb = (N + MB - 1) / MB;
+    EFIE_CUDA(cudaFuncSetAttribute(k_symv_multi<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)multi_smem<K>()));
+    k_symv_multi<K><<<std::min(ctx->num_sms, nb * nf), 256, multi_smem<K>(), ctx->stream>>>(d, t, N, nb, nf, xall, S, W,
+                                                                                           v0, ldw, ctl);
+    return efie_cuda_check(cudaGetLastError(), "snapshot products");
+}
+
+}  // namespace
+
+efie_status efie_snapshot_guess(efie_ctx *ctx, SolveWork &w, const void *Z, size_t zstride, const void *xall,
+                                const void *b, int nf, const SnapSpec &spec, void *x) {
+    cudaStream_t s = ctx->stream;
+    const int N = w.N, nblk = (N + 255) / 256;
+    int kmax = 0;
+    for (int f = 0; f < nf; f++) kmax = std::max(kmax, spec.k[f]);
+    if (nf < 1 || kmax < 1 || kmax > KMAX) return efie_fail(EFIE_ERR_ARGS, "snapshot guess: bad snapshot count");
+    // vectors per product launch; up to 15 snapshots go in one, more in two of twelve
+    const int ldw = kmax <= 4 ? 4 : kmax <= 8 ? 8 : kmax <= 12 ? 12 : kmax <= 15 ? 15 : 23;
+    const int QC = ldw <= 15 ? 16 : 24;
+    // W [nf][ldw][N], R [nf][nblk][QC][QC], coefficients [nf][KMAX], spec
+    const size_t nW = (size_t)nf * ldw * N, nR = (size_t)nf * nblk * QC * QC, nC = (size_t)nf * KMAX;
+    EFIE_TRY(w.snap.reserve(sizeof(double2) * (nW + nR + nC) + sizeof(SnapSpec)));
+    double2 *W = w.snap.as<double2>(), *R = W + nW, *coef = R + nR, *xd = static_cast<double2 *>(x);
+    int *dspec = reinterpret_cast<int *>(coef + nC);
+    EFIE_CUDA(cudaMemcpyAsync(dspec, &spec, sizeof(SnapSpec), cudaMemcpyHostToDevice, s));
+    const SnapIdx S{dspec, dspec + EFIE_MAX_BATCH};
+    const double2 *xa = static_cast<const double2 *>(xall), *bd = static_cast<const double2 *>(b);
+    CUtensorMap d, t;
+    EFIE_TRY(multi_maps(N, w.B, Z, zstride, &d, &t));
+    size_t tok = ctx->log.begin(s);
+    char *ctl = w.ctl.as<char>();
+    switch (ldw) {
+    case 4: EFIE_TRY(launch_multi<4>(ctx, d, t, N, nf, xa, S, W, 0, ldw, ctl)); break;
+    case 8: EFIE_TRY(launch_multi<8>(ctx, d, t, N, nf, xa, S, W, 0, ldw, ctl)); break;
+    case 12: EFIE_TRY(launch_multi<12>(ctx, d, t, N, nf, xa, S, W, 0, ldw, ctl)); break;
+    case 15: EFIE_TRY(launch_multi<16>(ctx, d, t, N, nf, xa, S, W, 0, ldw, ctl)); break;
+    default:
+        EFIE_TRY(launch_multi<12>(ctx, d, t, N, nf, xa, S, W, 0, ldw, ctl));
+        EFIE_TRY(launch_multi<12>(ctx, d, t, N, nf, xa, S, W, 12, ldw, ctl));
+    }
+    const int nprod = ldw > 15 ? 2 : 1;
+    ctx->log.end(EFIE_K_RESIDUAL, s, tok, nprod * 8.0 * (double)N * N * nf, nprod);
+    tok = ctx->log.begin(s);
+    const dim3 rows(nblk, nf);
+    if (QC == 16) {
+        k_tsqr_local<16><<<rows, 256, 0, s>>>(N, ldw, S.k, W, bd, R);
+        k_tsqr_combine<16><<<nf, 256, 0, s>>>(nblk, S.k, R, coef);
+    } else {
+        k_tsqr_local<24><<<rows, 256, 0, s>>>(N, ldw, S.k, W, bd, R);
+        k_tsqr_combine<24><<<nf, 256, 0, s>>>(nblk, S.k, R, coef);
+    }
+    k_snap_x<<<rows, 256, 0, s>>>(N, xa, S, coef, xd);
+    EFIE_CUDA(cudaGetLastError());
+    ctx->log.end(EFIE_K_OTHER, s, tok, 0.0, 3);
+    return EFIE_OK;
+}
+
+// Test entry: one guess from host arrays (Z column-major N x N, xs [k][N]).
+extern "C" efie_status efie_debug_snapshot_guess(efie_ctx *ctx, int32_t N, int32_t k, const efie_c128 *Z,
+                                                 const efie_c128 *xs, const efie_c128 *b, efie_c128 *x) {
+    if (!ctx || N < 1 || k < 1 || k > KMAX || !Z || !xs || !b || !x)
+        return efie_fail(EFIE_ERR_ARGS, "efie_debug_snapshot_guess: bad arguments");
+    DeviceGuard dg(ctx->device);
+    ctx->log.reset(false);
+    cudaStream_t s = ctx->stream;
+    SolveWork w;
+    w.N = N;
+    w.B = 1;
+    EFIE_TRY(w.ctl.reserve(64));
+    EFIE_CUDA(cudaMemsetAsync(w.ctl.p, 0, 64, s));
+    DevBuf dZ, dx, db, dg0;
+    const size_t v = sizeof(efie_c128) * (size_t)N;
+    EFIE_TRY(dZ.reserve(v * N));
+    EFIE_TRY(dx.reserve(v * k));
+    EFIE_TRY(db.reserve(v));
+    EFIE_TRY(dg0.reserve(v));
+    EFIE_CUDA(cudaMemcpyAsync(dZ.p, Z, v * N, cudaMemcpyHostToDevice, s));
+    EFIE_CUDA(cudaMemcpyAsync(dx.p, xs, v * k, cudaMemcpyHostToDevice, s));
+    EFIE_CUDA(cudaMemcpyAsync(db.p, b, v, cudaMemcpyHostToDevice, s));
+    SnapSpec sp{};
+    sp.k[0] = k;
+    for (int j = 0; j < k; j++) sp.pos[0][j] = j;
+    EFIE_TRY(efie_snapshot_guess(ctx, w, dZ.p, (size_t)N * N, dx.p, db.p, 1, sp, dg0.p));
+    int err = 0;
+    EFIE_CUDA(cudaMemcpyAsync(&err, w.ctl.as<char>() + 36, sizeof(int), cudaMemcpyDeviceToHost, s));
+    EFIE_CUDA(cudaMemcpyAsync(x, dg0.p, v, cudaMemcpyDeviceToHost, s));
+    EFIE_CUDA(cudaStreamSynchronize(s));
+    return err ? efie_fail(EFIE_ERR_TIMEOUT, "efie_debug_snapshot_guess: device error flag") : EFIE_OK;
+}

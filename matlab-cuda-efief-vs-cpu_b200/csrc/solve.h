@@ -6,6 +6,7 @@
 #include "efie_internal.h"
 
 constexpr int EFIE_MAX_BATCH = 64;
+constexpr int EFIE_SNAP_MAX = 23;   // snapshots an initial guess combines
 
 // Byte offset of element (row r, k) inside a K-major 64B-swizzled FP16 tile
 // (the tensor-core operand layout): 16-byte chunk (k / 8) XOR (r / 2) mod 4,
@@ -74,6 +75,7 @@ struct SolveWork {
     // gather): the factorization starts without converting Z
     bool planes_from_assembly = false;
     DevBuf spart;
+    DevBuf snap;   // products, R factors and coefficients of the snapshot guesses
     // look-ahead LU: the panel chain runs on `hi` (highest priority) while the
     // bulk of each deferred trailing update runs on `lo`
     cudaStream_t hi = nullptr, lo = nullptr;
@@ -149,6 +151,16 @@ struct GuessSpec {
     double w[3][EFIE_MAX_BATCH];
 };
 efie_status efie_interp_guess(efie_ctx *ctx, int N, int n, void *x, const void *xs, const GuessSpec &g);
+// x_f for the slots f < nf: the combination of the solved vectors
+// xall + N pos[f][j] (j < k[f], nearest frequency first) with the smallest
+// || b - Z_f x_f || (snapshot.cu).  Z symmetric (its upper triangle and
+// 128 x 128 diagonal blocks are read).
+struct SnapSpec {
+    int k[EFIE_MAX_BATCH];
+    int pos[EFIE_MAX_BATCH][EFIE_SNAP_MAX];
+};
+efie_status efie_snapshot_guess(efie_ctx *ctx, SolveWork &w, const void *Z, size_t zstride, const void *xall,
+                                const void *b, int nf, const SnapSpec &spec, void *x);
 efie_status efie_port_reduce(efie_ctx *ctx, int N, int B, const void *x, const double *wport, int model, int pe,
                              int ge, double V0, double Z0, void *out);
 
