@@ -110,7 +110,7 @@ __device__ __forceinline__ float2 crecip(float2 p, bool &zero) {
 __global__ void __launch_bounds__(256) k_diag_factor(int N, int k, int kb, int bi, float *__restrict__ planes,
                                                      size_t pstride, int ld, float2 *__restrict__ dinv,
                                                      size_t dstride, char *__restrict__ ctl,
-                                                     const int *__restrict__ active, int sym) {
+                                                     const int *__restrict__ active, int mirror) {
     const int f = blockIdx.x;
     if (!active[f]) return;
     extern __shared__ float2 dsm[];
@@ -128,8 +128,8 @@ __global__ void __launch_bounds__(256) k_diag_factor(int N, int k, int kb, int b
         const int r = e >> 6, c = e & 63;
         float2 v = make_float2(r == c ? 1.f : 0.f, 0.f);   // identity beyond kb
         if (r < kb && c < kb) {
-            // symmetric Z: the lower triangle, mirrored
-            const int rr = (sym && c > r) ? c : r, cc = (sym && c > r) ? r : c;
+            // mirror: the upper triangle from the lower one
+            const int rr = (mirror && c > r) ? c : r, cc = (mirror && c > r) ? r : c;
             const size_t o = (size_t)(k + rr) * ld + k + cc;
             v = make_float2(Ar[o], Ai[o]);
         }
@@ -155,18 +155,12 @@ __global__ void __launch_bounds__(256) k_diag_factor(int N, int k, int kb, int b
 #pragma unroll
             for (int j = 0; j < SB; j++) {
                 float2 u[SB];
-                // row o + j sits in lane j; symmetric Z (L D L^T): the row is
-                // the column below the pivot, row o + c in lane c
-                u[j] = shfl2(a0[j], j);
+                // row o + j sits in lane j
 #pragma unroll
-                for (int c = j + 1; c < SB; c++) u[c] = sym == 1 ? shfl2(a0[j], c) : shfl2(a0[c], j);
+                for (int c = j; c < SB; c++) u[c] = shfl2(a0[c], j);
                 bool z;
                 const float2 inv = crecip(u[j], z);
                 bad |= z;
-                if (sym == 1 && lane == j) {
-#pragma unroll
-                    for (int c = j + 1; c < SB; c++) a0[c] = u[c];
-                }
                 if (lane > j) {
                     const float2 l = cmulf(a0[j], inv);
                     a0[j] = l;
@@ -186,11 +180,7 @@ __global__ void __launch_bounds__(256) k_diag_factor(int N, int k, int kb, int b
         }
         __syncthreads();
         const int w = NB - o - SB;   // columns (rows) right of (below) the panel
-        if (sym == 1 && t < w) {     // U strip of L D L^T: U[o + i][c] = d_i L[c][o + i]
-            const int c = o + SB + t;
-#pragma unroll
-            for (int i = 0; i < SB; i++) A[o + i][c] = cmulf(A[o + i][o + i], A[c][o + i]);
-        } else if (t < w) {          // U strip: forward substitution with the panel's unit-lower block
+        if (t < w) {   // U strip: forward substitution with the panel's unit-lower block
             const int c = o + SB + t;
             float2 x[SB];
 #pragma unroll
@@ -283,16 +273,6 @@ __global__ void __launch_bounds__(256) k_diag_factor(int N, int k, int kb, int b
         __syncthreads();
     }
 
-    if (sym == 1) {
-        // U = D L^T: U^-1 = L^-T D^-1 from L^-1, so that U^-1 L^-1 is
-        // symmetric as the inverse of a symmetric block is
-        for (int e = t; e < NB * NB; e += 256) {
-            const int r = e >> 6, c = e & 63;
-            bool z;
-            Y[r][c] = r <= c ? cmulf(X[c][r], crecip(A[c][c], z)) : make_float2(0.f, 0.f);
-        }
-        __syncthreads();
-    }
     // ---- factors back to the planes, inverses to their slots ----
     for (int e = t; e < NB * NB; e += 256) {
         const int r = e >> 6, c = e & 63;
@@ -305,6 +285,172 @@ __global__ void __launch_bounds__(256) k_diag_factor(int N, int k, int kb, int b
         Uinv[e] = Y[r][c];
     }
     if (t == 0 && bad) atomicExch(err, 1);
+}
+
+// ---------------------------------------------------------------------------
+// The same for a symmetric Z (L D L^T from the block's lower triangle), the
+// launch every panel of a sweep waits for.  Bound by latency: one CTA per
+// frequency, its steps in sequence.  Fully unrolled register panels (the
+// general kernel above) run 80 KB of straight-line code once per launch, most
+// of it instruction fetches; here every step is a short loop over 16-wide
+// blocks on all 256 threads, one element of a 16 x 16 block each:
+//   A_pp = L D L^T by 16 rank-1 steps, X_pp = L_pp^-1 carried along as the
+//   right-hand side, one barrier per step (the pivot row in two buffers);
+//   V = A_rp X_pp^T for the rows r below (U_pr = V^T), L_rp = V D^-1;
+//   A_rc -= L_rp U_pc on the 16 x 16 blocks of the lower triangle;
+// then the off-diagonal blocks of X = L^-1 by block diagonals,
+//   X_ij = -X_ii sum_{j <= m < i} L_im X_mj,
+// and U^-1 = X^T D^-1, so that U^-1 L^-1 is symmetric as the inverse of a
+// symmetric block is.
+// ---------------------------------------------------------------------------
+constexpr size_t kDiagSymSmem = sizeof(float2) * (2 * NB * (NB + 1) + 3 * SB * (SB + 1) + 4 * SB + NB);
+
+__global__ void __launch_bounds__(256) k_diag_sym(int N, int k, int kb, int bi, float *__restrict__ planes,
+                                                  size_t pstride, int ld, float2 *__restrict__ dinv, size_t dstride,
+                                                  char *__restrict__ ctl, const int *__restrict__ active) {
+    const int f = blockIdx.x;
+    if (!active[f]) return;
+    extern __shared__ float2 dsm[];
+    float2(*A)[NB + 1] = reinterpret_cast<float2(*)[NB + 1]>(dsm);   // lower triangle, then L\U
+    float2(*X)[NB + 1] = A + NB;                                      // L^-1
+    float2(*T)[SB][SB + 1] = reinterpret_cast<float2(*)[SB][SB + 1]>(dsm + 2 * NB * (NB + 1));
+    float2 *prow = dsm + 2 * NB * (NB + 1) + 3 * SB * (SB + 1);      // pivot rows of A and X, two buffers
+    float2 *rd = prow + 4 * SB;                                       // 1 / d
+    float *Ar = planes + pstride * f, *Ai = Ar + (size_t)ld * N;
+    float2 *Linv = dinv + dstride * f + (size_t)bi * 2 * NB * NB, *Uinv = Linv + NB * NB;
+    const int t = threadIdx.x, i = t >> 4, c = t & 15;
+#pragma unroll 8
+    for (int e = t; e < NB * NB; e += 256) {
+        const int r = e >> 6, q = e & 63;
+        float2 v = make_float2(r == q ? 1.f : 0.f, 0.f);   // identity beyond kb
+        if (r < kb && q <= r) {
+            const size_t o = (size_t)(k + r) * ld + k + q;
+            v = make_float2(Ar[o], Ai[o]);
+        }
+        A[r][q] = v;
+        X[r][q] = make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    bool bad = false;
+#pragma unroll 1
+    for (int p = 0; p < NB / SB; p++) {
+        const int o = p * SB;
+        // 16 x 16 diagonal block: this thread's element (both triangles kept) and that of X_pp
+        float2 a = i >= c ? A[o + i][o + c] : A[o + c][o + i];
+        float2 x = make_float2(i == c ? 1.f : 0.f, 0.f);
+        float2 out = a;   // U on and above the diagonal, L below
+#pragma unroll 2
+        for (int j = 0; j < SB; j++) {
+            float2 *u = prow + (j & 1) * 2 * SB, *xr = u + SB;
+            if (i == j) {
+                u[c] = a;
+                xr[c] = x;
+                if (c >= j) out = a;
+            }
+            __syncthreads();
+            bool z;
+            const float2 inv = crecip(u[j], z);
+            bad |= z;
+            if (i > j) {
+                const float2 l = cmulf(u[i], inv);   // the column below the pivot is the row right of it
+                if (c == j) out = l;
+                cfms(a, l, u[c]);
+                cfms(x, l, xr[c]);
+            } else if (i == j && c == j) {
+                rd[o + j] = inv;
+            }
+        }
+        A[o + i][o + c] = out;
+        X[o + i][o + c] = x;
+        __syncthreads();
+        const int nr = NB / SB - 1 - p;   // 16-row blocks below
+        float2 v[3];
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            if (b >= nr) break;
+            const float2 *row = A[o + SB * (b + 1) + i] + o;
+            float2 s = make_float2(0.f, 0.f);
+#pragma unroll 4
+            for (int m = 0; m < SB; m++) cfma(s, row[m], X[o + c][o + m]);
+            v[b] = s;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            if (b >= nr) break;
+            const int r = o + SB * (b + 1) + i;
+            A[o + c][r] = v[b];
+            A[r][o + c] = cmulf(v[b], rd[o + c]);
+        }
+        __syncthreads();
+        // trailing blocks on and below the diagonal: rows i + 16 a, columns c + 16 b
+        float2 acc[3][3];
+#pragma unroll
+        for (int y = 0; y < 3; y++)
+#pragma unroll
+            for (int b = 0; b < 3; b++) acc[y][b] = make_float2(0.f, 0.f);
+#pragma unroll 2
+        for (int m = 0; m < SB; m++) {
+            float2 l[3], u[3];
+#pragma unroll
+            for (int y = 0; y < 3; y++)
+                if (y < nr) {
+                    l[y] = A[o + SB * (y + 1) + i][o + m];
+                    u[y] = A[o + m][o + SB * (y + 1) + c];
+                }
+#pragma unroll
+            for (int y = 0; y < 3; y++)
+#pragma unroll
+                for (int b = 0; b <= y; b++)
+                    if (y < nr) cfma(acc[y][b], l[y], u[b]);
+        }
+#pragma unroll
+        for (int y = 0; y < 3; y++)
+#pragma unroll
+            for (int b = 0; b <= y; b++)
+                if (y < nr) {
+                    float2 &e = A[o + SB * (y + 1) + i][o + SB * (b + 1) + c];
+                    // above the diagonal of a diagonal block nothing is read before it is overwritten
+                    e.x -= acc[y][b].x;
+                    e.y -= acc[y][b].y;
+                }
+        __syncthreads();
+    }
+    // off-diagonal blocks of X by block diagonals r
+#pragma unroll 1
+    for (int r = 1; r < NB / SB; r++) {
+        const int n = NB / SB - r;
+#pragma unroll 1
+        for (int j = 0; j < n; j++) {
+            const int I = j + r;
+            float2 s = make_float2(0.f, 0.f);
+#pragma unroll 4
+            for (int m = j * SB; m < I * SB; m++) cfma(s, A[I * SB + i][m], X[m][j * SB + c]);
+            T[j][i][c] = s;
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int j = 0; j < n; j++) {
+            const int I = j + r;
+            float2 s = make_float2(0.f, 0.f);
+#pragma unroll 4
+            for (int m = 0; m < SB; m++) cfms(s, X[I * SB + i][I * SB + m], T[j][m][c]);
+            X[I * SB + i][j * SB + c] = s;
+        }
+        __syncthreads();
+    }
+#pragma unroll 4
+    for (int e = t; e < NB * NB; e += 256) {
+        const int r = e >> 6, q = e & 63;
+        if (r < kb && q < kb) {
+            const size_t o = (size_t)(k + r) * ld + k + q;
+            Ar[o] = A[r][q].x;
+            Ai[o] = A[r][q].y;
+        }
+        Linv[e] = X[r][q];
+        Uinv[e] = r <= q ? cmulf(X[q][r], rd[q]) : make_float2(0.f, 0.f);
+    }
+    if (t == 0 && bad) atomicExch(reinterpret_cast<int *>(ctl + 64 * f + 36), 1);
 }
 
 // A finished 64 x 64 factor block (thread (ty, tx) holds rows ty + 16 a,
@@ -831,6 +977,7 @@ efie_status set_smem_attrs() {
     if (done) return EFIE_OK;
     EFIE_CUDA(cudaFuncSetAttribute(k_panels, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmem));
     EFIE_CUDA(cudaFuncSetAttribute(k_diag_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSmem));
+    EFIE_CUDA(cudaFuncSetAttribute(k_diag_sym, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDiagSymSmem));
     EFIE_CUDA(cudaFuncSetAttribute(k_update_simt, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTwoTiles));
     done = true;
     return EFIE_OK;
@@ -982,8 +1129,12 @@ efie_status efie_mixed_factor_launch(efie_ctx *ctx, SolveWork &w, const void *Z,
                     const int s1 = k + kb, rest = N - s1;
                     const bool inpanel = s1 < He;
                     tok = log.begin(s);
-                    k_diag_factor<<<B, 256, kDiagSmem, s>>>(N, k, kb, bi, planes, w.pstride, ld, dinv, w.dstride, ctl,
-                                                            active, sym ? (g_sym_lu_disabled == 3 ? 2 : 1) : 0);
+                    if (sym && g_sym_lu_disabled != 3)
+                        k_diag_sym<<<B, 256, kDiagSymSmem, s>>>(N, k, kb, bi, planes, w.pstride, ld, dinv, w.dstride,
+                                                                ctl, active);
+                    else
+                        k_diag_factor<<<B, 256, kDiagSmem, s>>>(N, k, kb, bi, planes, w.pstride, ld, dinv, w.dstride,
+                                                                ctl, active, sym ? 1 : 0);
                     if (rest > 0) {
                         dim3 pg((rest + NB - 1) / NB, sym ? 1 : 2, B);
                         k_panels<<<pg, 256, kPanelSmem, s>>>(N, k, kb, bi, planes, w.pstride, ld, dinv, w.dstride,
