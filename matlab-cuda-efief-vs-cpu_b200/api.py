@@ -217,7 +217,7 @@ def ggassemble_ZV_EFIE_RWG_DIFF_GPU_FAST(*args, nargout=2):
     m = _Marshal()
     mesh = m.mesh(V, F, E, pt, mt, ps, ms, rp, rm, Ap, Am, ln)
     pp = m.prepack(pre, Nt)
-    Z = np.zeros((Ne, Ne), dtype=np.complex128, order="F")
+    Z = np.empty((Ne, Ne), dtype=np.complex128, order="F")   # the call writes all of it
     Vr = np.zeros(Ne, dtype=np.complex128)
     ex = np.ascontiguousarray(excv[:4])
     nat.check(nat.lib().efie_ggassemble_zv(nat.context(), C.byref(mesh), C.byref(pp), _cscalar(k),
@@ -242,7 +242,7 @@ def gassemble_ZV_EFIE_RWG_DIFF_GPU_FAST(*args, nargout=2):
     _port_check(int(excv[0]), int(excv[1]), Ne)
     m = _Marshal()
     mesh = m.mesh(V, F, E, pt, mt, ps, ms, rp, rm, Ap, Am, ln)
-    Z = np.zeros((Ne, Ne), dtype=np.complex128, order="F")
+    Z = np.empty((Ne, Ne), dtype=np.complex128, order="F")   # the call writes all of it
     Vr = np.zeros(Ne, dtype=np.complex128)
     ex = np.ascontiguousarray(excv[:5])
     nat.check(nat.lib().efie_gassemble_zv(nat.context(), C.byref(mesh), _cscalar(k), float(_scalar(omega)),

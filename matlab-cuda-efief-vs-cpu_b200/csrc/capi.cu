@@ -1,10 +1,12 @@
 // C ABI of libefie_b200: argument checks that mirror the reference MEX
 // functions, host-side RHS, plans and frequency sweeps.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <new>
 #include <string>
+#include <thread>
 #include <map>
 #include <mutex>
 #include <vector>
@@ -119,6 +121,7 @@ extern "C" void efie_ctx_destroy(efie_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->solver) cusolverDnDestroy(ctx->solver);
     ctx->status.release();
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     efie_pool_trim(ctx->device);
     delete ctx;
@@ -336,6 +339,109 @@ efie_status check_eps(double omega, efie_c128 eps) {
 
 }  // namespace
 
+namespace {
+
+// A large result to pageable host memory.  cudaMemcpy stages such a copy
+// through one thread, which also takes the page faults of a fresh array (Ne
+// 3086, 152 MB: 35 ms, 4.3 GB/s).  Here pieces of 2 MB -- on the destination's
+// 2 MB boundaries, so that no two threads fault on one huge page -- land in
+// pinned buffers while several threads copy the ones before out, a whole piece
+// each.  The pinned buffers (48 MB; allocating them takes 45 ms) stay with the
+// context, the threads end with the call; small results, pinned destinations
+// and any failure to set up take the plain copy.
+constexpr size_t kPiece = (size_t)2 << 20;
+constexpr int kCopyBufs = 24;
+constexpr size_t kCopyMin = (size_t)8 << 20;   // below it the threads cost more than they save
+
+struct HostCopy {
+    cudaEvent_t ev[kCopyBufs] = {};
+    std::vector<std::thread> threads;
+    std::atomic<int64_t> ready{0};             // pieces in their pinned buffers (-1: stop)
+    std::atomic<int64_t> out[kCopyBufs];       // the last piece copied out of each buffer
+    ~HostCopy() {
+        for (std::thread &t : threads) t.join();
+        for (cudaEvent_t e : ev)
+            if (e) cudaEventDestroy(e);
+    }
+};
+
+efie_status copy_to_host(efie_ctx *ctx, void *dst, const void *src, size_t bytes) {
+    cudaStream_t s = ctx->stream;
+    cudaPointerAttributes at{};
+    const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    const int nt = (int)std::min(12u, std::thread::hardware_concurrency() * 3 / 4);
+    HostCopy hc;
+    bool ok = bytes >= kCopyMin && pageable && nt > 1;
+    if (ok && !ctx->pinned && cudaHostAlloc(&ctx->pinned, kPiece * kCopyBufs, cudaHostAllocDefault) != cudaSuccess) {
+        ctx->pinned = nullptr;
+        ok = false;
+    }
+    char *const pinned = static_cast<char *>(ctx->pinned);
+    for (int b = 0; ok && b < kCopyBufs; b++) {
+        ok = cudaEventCreateWithFlags(&hc.ev[b], cudaEventDisableTiming) == cudaSuccess;
+        hc.out[b].store(b - kCopyBufs);
+    }
+    // piece i covers [begin(i), begin(i + 1)) of the result
+    const size_t head = (kPiece - reinterpret_cast<uintptr_t>(dst) % kPiece) % kPiece;
+    const int64_t n = (int64_t)((bytes - std::min(bytes, head) + kPiece - 1) / kPiece) + (head > 0);
+    auto begin = [=](int64_t i) -> size_t {
+        return i <= 0 ? 0 : std::min(bytes, head > 0 ? head + (size_t)(i - 1) * kPiece : (size_t)i * kPiece);
+    };
+    if (ok) {
+        try {
+            for (int t = 0; t < nt; t++)
+                hc.threads.emplace_back([&hc, begin, pinned, t, nt, n, dst] {
+                    for (int64_t i = t; i < n; i += nt) {
+                        int64_t r;
+                        while ((r = hc.ready.load(std::memory_order_acquire)) >= 0 && r <= i) std::this_thread::yield();
+                        if (r < 0) return;
+                        const size_t off = begin(i);
+                        std::memcpy(static_cast<char *>(dst) + off, pinned + (i % kCopyBufs) * kPiece, begin(i + 1) - off);
+                        hc.out[i % kCopyBufs].store(i, std::memory_order_release);
+                    }
+                });
+        } catch (...) {   // no threads to be had
+            hc.ready.store(-1);
+            ok = false;
+        }
+    }
+    if (!ok) {
+        cudaGetLastError();
+        EFIE_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
+        EFIE_CUDA(cudaStreamSynchronize(s));
+        return EFIE_OK;
+    }
+    cudaError_t e = cudaSuccess;
+    int64_t fetched = 0, handed = 0;
+    while (handed < n && e == cudaSuccess) {
+        // fetch while buffers are free (their previous piece is out), then hand over the oldest in flight
+        while (fetched < n && e == cudaSuccess &&
+               hc.out[fetched % kCopyBufs].load(std::memory_order_acquire) == fetched - kCopyBufs) {
+            const int b = (int)(fetched % kCopyBufs);
+            const size_t off = begin(fetched);
+            e = cudaMemcpyAsync(pinned + b * kPiece, static_cast<const char *>(src) + off, begin(fetched + 1) - off,
+                                cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaEventRecord(hc.ev[b], s);
+            fetched++;
+        }
+        if (handed < fetched && e == cudaSuccess) {
+            e = cudaEventSynchronize(hc.ev[handed % kCopyBufs]);
+            if (e == cudaSuccess) hc.ready.store(++handed, std::memory_order_release);
+        } else {
+            std::this_thread::yield();
+        }
+    }
+    if (e != cudaSuccess) {
+        hc.ready.store(-1);
+        cudaStreamSynchronize(s);   // copies in flight write the pinned buffers
+        return efie_fail(EFIE_ERR_CUDA, std::string("copy to host: ") + cudaGetErrorString(e));
+    }
+    return EFIE_OK;   // ~HostCopy joins the threads
+}
+
+}  // namespace
+
 // ---------------------------------------------------------------------------
 // Assembly-only entry points
 // ---------------------------------------------------------------------------
@@ -360,8 +466,7 @@ extern "C" efie_status efie_ggassemble_zv(efie_ctx *ctx, const efie_mesh *mesh, 
     DevBuf dZ;
     EFIE_TRY(dZ.reserve(sizeof(efie_c128) * (size_t)Ne * Ne));
     EFIE_TRY(efie_assemble_device(ctx, g, ph, dZ.p));
-    EFIE_CUDA(cudaMemcpyAsync(Z, dZ.p, sizeof(efie_c128) * (size_t)Ne * Ne, cudaMemcpyDeviceToHost, ctx->stream));
-    EFIE_CUDA(cudaStreamSynchronize(ctx->stream));
+    EFIE_TRY(copy_to_host(ctx, Z, dZ.p, sizeof(efie_c128) * (size_t)Ne * Ne));
     for (int e = 0; e < Ne; e++) Vrhs[e] = efie_c128{rhs[e], 0.0};
     return EFIE_OK;
 }
@@ -384,8 +489,7 @@ extern "C" efie_status efie_gassemble_zv(efie_ctx *ctx, const efie_mesh *mesh, e
     DevBuf dZ, scratch;
     EFIE_TRY(dZ.reserve(sizeof(efie_c128) * (size_t)Ne * Ne));
     EFIE_TRY(efie_assemble_centroid_device(ctx, mesh, exc[4], ph, dZ.p, scratch));
-    EFIE_CUDA(cudaMemcpyAsync(Z, dZ.p, sizeof(efie_c128) * (size_t)Ne * Ne, cudaMemcpyDeviceToHost, ctx->stream));
-    EFIE_CUDA(cudaStreamSynchronize(ctx->stream));
+    EFIE_TRY(copy_to_host(ctx, Z, dZ.p, sizeof(efie_c128) * (size_t)Ne * Ne));
     for (int e = 0; e < Ne; e++) Vrhs[e] = efie_c128{rhs[e], 0.0};
     return EFIE_OK;
 }

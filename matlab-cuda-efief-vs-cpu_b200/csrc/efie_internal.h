@@ -145,6 +145,7 @@ struct efie_ctx {
     cusolverDnHandle_t solver = nullptr;
     int num_sms = 0;
     int cc_major = 0;
+    void *pinned = nullptr;   // staging of large results to pageable host memory (copy_to_host)
     DevBuf status;   // device-side error flags of bounded waits (int32[8])
     KernelLog log;
 };
