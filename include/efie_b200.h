@@ -170,7 +170,7 @@ typedef struct efie_sweep_opts {
     int32_t refine_method;   /* efie_refine_method; default EFIE_REFINE_GMRES    */
     int32_t graphs;          /* 1 (default): with timing off, the mixed LU of a
                                 batch replays a CUDA graph captured on the
-                                plan's first batch; 0: eager launches        */
+                                plan's second batch; 0: eager launches       */
     int32_t tile_chain;      /* complex columns of the tensor-core tile of the LU's
                                 K = 64 panel-chain updates: 128 or 256 (0 = tuned) */
     int32_t tile_bulk;       /* ... of the outer panels' trailing updates (0 = tuned) */

@@ -883,13 +883,13 @@ __global__ void __launch_bounds__(256) k_centroid_z(int Ne, const Side *__restri
 }
 
 // The pair mask (1 = near, adjacent or self: not a regular pair) from the
-// pair list, on a zeroed mask: entry (t1, t2) and, for a symmetric list, (t2, t1).
-__global__ void k_mask_pairs(int Nt, int n, const int2 *__restrict__ list, bool both, uint8_t *__restrict__ mask) {
+// pair list, on a zeroed mask: entries (t1, t2) and (t2, t1).
+__global__ void k_mask_pairs(int Nt, int n, const int2 *__restrict__ list, uint8_t *__restrict__ mask) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int2 pr = list[i];
     mask[(size_t)pr.x + (size_t)Nt * pr.y] = 1;
-    if (both) mask[(size_t)pr.y + (size_t)Nt * pr.x] = 1;
+    mask[(size_t)pr.y + (size_t)Nt * pr.x] = 1;
 }
 
 __global__ void k_mask_self(int Nt, uint8_t *__restrict__ mask) {
@@ -921,6 +921,39 @@ Physics efie_physics(double freq, double mu, efie_c128 eps) {
     efie_c128 k = {omega * (sr * std::cos(half)), omega * (sr * std::sin(half))};
     return efie_physics_k(k, omega, mu, eps);
 }
+
+namespace {
+
+// Points and weights of a cache in the boundary layout (r [n x 3 x ns x Nt],
+// w [n x ns x Nt]) to points relative to the triangles' origins with the
+// weight in the fourth lane: pts[(t ns + p) n + i].
+__global__ void __launch_bounds__(256) k_pack_points(int n, int ns, size_t total, const double *__restrict__ r,
+                                                     const double *__restrict__ w,
+                                                     const double4 *__restrict__ origin, double4 *__restrict__ pts) {
+    const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;   // = (t ns + p) n + i, the order of w
+    if (q >= total) return;
+    const size_t tp = q / n, t = tp / ns;
+    const int i = (int)(q - tp * n);
+    const double4 o = origin[t];
+    const double *v = r + tp * 3 * n + i;
+    pts[q] = make_double4(v[0] - o.x, v[n] - o.y, v[2 * n] - o.z, w[q]);
+}
+
+// `raw` stages the two arrays; it may be reused once the stream has run the kernel
+efie_status pack_points(efie_ctx *ctx, DevBuf &raw, const double *r, const double *w, int n, int ns, int Nt,
+                        const DevBuf &origin, DevBuf &pts) {
+    cudaStream_t s = ctx->stream;
+    const size_t total = (size_t)Nt * ns * n;
+    EFIE_TRY(raw.reserve(sizeof(double) * 4 * total));
+    double *dr = raw.as<double>(), *dw = dr + 3 * total;
+    EFIE_CUDA(cudaMemcpyAsync(dr, r, sizeof(double) * 3 * total, cudaMemcpyHostToDevice, s));
+    EFIE_CUDA(cudaMemcpyAsync(dw, w, sizeof(double) * total, cudaMemcpyHostToDevice, s));
+    k_pack_points<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(n, ns, total, dr, dw, origin.as<double4>(),
+                                                                 pts.as<double4>());
+    return efie_cuda_check(cudaGetLastError(), "pack_points");
+}
+
+}  // namespace
 
 // Host-side repacking of the boundary arrays into the device layout.
 efie_status efie_geom_upload(efie_ctx *ctx, const efie_mesh *mesh, const efie_prepack *pre, int scheme,
@@ -1011,9 +1044,7 @@ efie_status efie_geom_upload(efie_ctx *ctx, const efie_mesh *mesh, const efie_pr
         }
     }
 
-    // the pair list whose entries (and diagonal) the device mask marks
     std::vector<int2> list;
-    bool mask_both = true;
     if (scheme == EFIE_SCHEME_REF && !pre) {
         // caches and near-pair list computed on the device from V/F (precompute.cu)
         EFIE_TRY(efie_geom_precompute_device(ctx, mesh, popts, g));
@@ -1023,65 +1054,16 @@ efie_status efie_geom_upload(efie_ctx *ctx, const efie_mesh *mesh, const efie_pr
         g.Nq2 = Nq2;
         g.NsS = NsS;
         g.NsN = NsN;
-        std::vector<double4> reg((size_t)Nt * Nq), nearp((size_t)Nt * NsN * Nq2), selfp((size_t)Nt * NsS * Nq2);
-        for (int t = 0; t < Nt; t++) {
-            const double4 o = origin[t];
-            for (int i = 0; i < Nq; i++) {
-                const double *r = pre->r_reg + i + (size_t)Nq * 3 * t;
-                reg[(size_t)t * Nq + i] = make_double4(r[0] - o.x, r[Nq] - o.y, r[2 * Nq] - o.z,
-                                                       pre->w_reg[i + (size_t)Nq * t]);
-            }
-            for (int p = 0; p < NsN; p++)
-                for (int i = 0; i < Nq2; i++) {
-                    const double *r = pre->near_r + i + (size_t)Nq2 * 3 * p + (size_t)Nq2 * 3 * NsN * t;
-                    nearp[((size_t)t * NsN + p) * Nq2 + i] =
-                        make_double4(r[0] - o.x, r[Nq2] - o.y, r[2 * Nq2] - o.z,
-                                     pre->near_w[i + (size_t)Nq2 * p + (size_t)Nq2 * NsN * t]);
-                }
-            for (int p = 0; p < NsS; p++)
-                for (int i = 0; i < Nq2; i++) {
-                    const double *r = pre->self_r + i + (size_t)Nq2 * 3 * p + (size_t)Nq2 * 3 * NsS * t;
-                    selfp[((size_t)t * NsS + p) * Nq2 + i] =
-                        make_double4(r[0] - o.x, r[Nq2] - o.y, r[2 * Nq2] - o.z,
-                                     pre->self_w[i + (size_t)Nq2 * p + (size_t)Nq2 * NsS * t]);
-                }
-        }
-        EFIE_TRY(up(g.reg_pts, reg.data(), sizeof(double4) * reg.size()));
-        EFIE_TRY(up(g.near_pts, nearp.data(), sizeof(double4) * nearp.size()));
-        EFIE_TRY(up(g.self_pts, selfp.data(), sizeof(double4) * selfp.size()));
+        EFIE_TRY(g.reg_pts.reserve(sizeof(double4) * (size_t)Nt * Nq));
+        EFIE_TRY(g.near_pts.reserve(sizeof(double4) * (size_t)Nt * NsN * Nq2));
+        EFIE_TRY(g.self_pts.reserve(sizeof(double4) * (size_t)Nt * NsS * Nq2));
         EFIE_TRY(up(g.self_a, pre->self_a, sizeof(double) * (size_t)Nt * NsS));
         EFIE_TRY(up(g.aeq, pre->aeqTri, sizeof(double) * Nt));
-        // near pairs (t1 != t2, nearMat nonzero) column by column, skipping
-        // zero bytes eight at a time: nearMat is almost all zeros
-        std::vector<int2> all;
-        for (int t2 = 0; t2 < Nt; t2++) {
-            const uint8_t *col = pre->nearMat + (size_t)Nt * t2;
-            int t1 = 0;
-            for (; t1 + 8 <= Nt; t1 += 8) {
-                uint64_t w;
-                std::memcpy(&w, col + t1, 8);
-                if (!w) continue;
-                for (int j = 0; j < 8; j++)
-                    if (col[t1 + j] && t1 + j != t2) all.push_back(make_int2(t1 + j, t2));
-            }
-            for (; t1 < Nt; t1++)
-                if (col[t1] && t1 != t2) all.push_back(make_int2(t1, t2));
-        }
-        // pair regimes; symmetric storage only if nearMat is symmetric: every
-        // (t1, t2) of the list has its (t2, t1)
-        std::vector<int64_t> keys(all.size());
-        for (size_t i = 0; i < all.size(); i++) keys[i] = (int64_t)all[i].x * Nt + all[i].y;
-        std::sort(keys.begin(), keys.end());
-        bool sym = true;
-        for (size_t i = 0; i < all.size() && sym; i++)
-            sym = std::binary_search(keys.begin(), keys.end(), (int64_t)all[i].y * Nt + all[i].x);
-        g.symmetric = sym;
-        // the near list in column order (t1 < t2 when symmetric)
-        for (const int2 &pr : all)
-            if (!sym || pr.x < pr.y) list.push_back(pr);
-        mask_both = sym;
-        g.n_near = (int)list.size();
-        EFIE_TRY(up(g.near_list, list.data(), sizeof(int2) * (list.empty() ? 1 : list.size())));
+        DevBuf raw;
+        EFIE_TRY(pack_points(ctx, raw, pre->r_reg, pre->w_reg, Nq, 1, Nt, g.origin, g.reg_pts));
+        EFIE_TRY(pack_points(ctx, raw, pre->near_r, pre->near_w, Nq2, NsN, Nt, g.origin, g.near_pts));
+        EFIE_TRY(pack_points(ctx, raw, pre->self_r, pre->self_w, Nq2, NsS, Nt, g.origin, g.self_pts));
+        EFIE_TRY(efie_geom_near_device(ctx, pre->nearMat, Nt, g));
     } else if (scheme == EFIE_SCHEME_EXTRACT) {
         // rule points of every triangle from V/F (map_ref_to_vertices.m form), weights times 2A
         const int order = rule_order ? rule_order : EFIE_QUAD_DUNAVANT7;
@@ -1134,16 +1116,16 @@ efie_status efie_geom_upload(efie_ctx *ctx, const efie_mesh *mesh, const efie_pr
         return efie_fail(EFIE_ERR_ARGS, "unknown scheme");
     }
     // the pair mask is built on the device from the list: zeros, the list's
-    // entries (both orientations when symmetric), the diagonal
-    {
+    // entries (both orientations when symmetric), the diagonal; a prepack's
+    // nearMat has become the mask already
+    if (scheme != EFIE_SCHEME_REF || !pre) {
         const size_t nn = (size_t)Nt * Nt;
         EFIE_TRY(g.near_mask.reserve(nn));
         EFIE_CUDA(cudaMemsetAsync(g.near_mask.p, 0, nn, ctx->stream));
         DevBuf &lst = scheme == EFIE_SCHEME_REF ? g.near_list : g.adj_list;
         const int n = scheme == EFIE_SCHEME_REF ? g.n_near : g.n_adj;
         if (n > 0)
-            k_mask_pairs<<<(n + 255) / 256, 256, 0, ctx->stream>>>(Nt, n, lst.as<int2>(), mask_both,
-                                                                   g.near_mask.as<uint8_t>());
+            k_mask_pairs<<<(n + 255) / 256, 256, 0, ctx->stream>>>(Nt, n, lst.as<int2>(), g.near_mask.as<uint8_t>());
         k_mask_self<<<(Nt + 255) / 256, 256, 0, ctx->stream>>>(Nt, g.near_mask.as<uint8_t>());
         EFIE_CUDA(cudaGetLastError());
     }

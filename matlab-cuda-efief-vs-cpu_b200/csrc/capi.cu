@@ -191,9 +191,13 @@ void *efie_pool_get(size_t n, size_t *got, cudaError_t *err) {
     return p;
 }
 
+// set while the device has been synchronised for everything this thread
+// releases: a plan's thirty-odd buffers then wait once, not once each
+static thread_local bool t_pool_synced = false;
+
 void efie_pool_put(void *p, size_t bytes) {
     // the block's last users may still run: finish them as cudaFree would
-    cudaDeviceSynchronize();
+    if (!t_pool_synced) cudaDeviceSynchronize();
     int dev = 0;
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lk(g_pool_mu);
@@ -521,8 +525,9 @@ struct efie_plan {
     DevBuf xall;   // solutions of a sweep by sorted frequency (initial guesses of later batches)
     int lwork_elems = -1;
     SolveWork sw;
-    // the mixed factorization as a CUDA graph (captured on the first untimed
+    // the mixed factorization as a CUDA graph (captured on the second untimed
     // batch, replayed for every later one) and its per-class launch counts
+    bool factored = false;
     cudaGraphExec_t factor_graph = nullptr;
     int graph_launches[EFIE_NUM_KERNEL_CLASSES] = {0};
     double graph_work[EFIE_NUM_KERNEL_CLASSES] = {0};
@@ -541,8 +546,12 @@ efie_status plan_factor(efie_plan *p, const int *active, int nact) {
     efie_ctx *ctx = p->ctx;
     const size_t NN = (size_t)p->Ne * p->Ne;
     EFIE_TRY(efie_mixed_factor_prepare(ctx, p->sw, active));
-    // the legacy default stream cannot be captured: launch eagerly there
-    const bool graph = !ctx->log.timing && p->opts.graphs && ctx->stream != nullptr;
+    // the legacy default stream cannot be captured: launch eagerly there; a
+    // plan's first factorization runs eagerly too: capturing and instantiating
+    // (0.7 ms at Ne 538) repay themselves from the second replay on, and a
+    // one-call sweep factors once
+    const bool graph = !ctx->log.timing && p->opts.graphs && ctx->stream != nullptr && p->factored;
+    p->factored = true;
     if (!graph) return efie_mixed_factor_launch(ctx, p->sw, p->Z.p, NN, nact);
     KernelLog &log = ctx->log;
     if (!p->factor_graph) {
@@ -811,8 +820,10 @@ extern "C" efie_status efie_plan_set_timing(efie_plan *p, int32_t timing) {
 extern "C" void efie_plan_destroy(efie_plan *p) {
     if (!p) return;
     DeviceGuard dg(p->ctx->device);
-    cudaStreamSynchronize(p->ctx->stream);
+    cudaDeviceSynchronize();   // the plan's work, on all its streams
+    t_pool_synced = true;
     delete p;
+    t_pool_synced = false;
 }
 
 // Initial guess of the frequency at sorted position q: the Lagrange

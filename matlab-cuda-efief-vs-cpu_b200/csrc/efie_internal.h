@@ -212,6 +212,8 @@ efie_status efie_z_mirror(efie_ctx *ctx, void *Z, int Ne);
 // into the plan's layout (origins, cache points, near-pair list)
 efie_status efie_geom_precompute_device(efie_ctx *ctx, const efie_mesh *mesh, const efie_precompute_opts *o,
                                         GeomDev &g);
+// the near-pair list, the pair mask and g.symmetric from a host nearMat [Nt x Nt]
+efie_status efie_geom_near_device(efie_ctx *ctx, const uint8_t *nearMat, int Nt, GeomDev &g);
 // pr (optional, symmetric gather only): also write the complex64 working
 // matrix of the mixed solver as FP32 planes, re at pr[m * ld + n], im at
 // pr[(Ne + m) * ld + n]

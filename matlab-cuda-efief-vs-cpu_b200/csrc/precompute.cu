@@ -207,6 +207,59 @@ __global__ void __launch_bounds__(256) k_near_pairs(int Nt, const double4 *__res
     if (!list && tid == 0) count[t2] = total;
 }
 
+// Pairs of column t2 from a near matrix given as bytes (column-major): the
+// entries t1 < t2 of a symmetric one, every t1 != t2 otherwise.
+__global__ void __launch_bounds__(256) k_mat_pairs(int Nt, const uint8_t *__restrict__ nm, const int *__restrict__ asym,
+                                                   int *__restrict__ count, const long long *__restrict__ offset,
+                                                   int2 *__restrict__ list) {
+    __shared__ int warp_n[8];
+    const int t2 = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int end = *asym ? Nt : t2;
+    long long base = list ? offset[t2] : 0;
+    int total = 0;
+    for (int c0 = 0; c0 < end; c0 += 256) {
+        const int t1 = c0 + tid;
+        const bool nr = t1 < end && t1 != t2 && nm[(size_t)t1 + (size_t)Nt * t2];
+        const unsigned bal = __ballot_sync(0xffffffffu, nr);
+        if (lane == 0) warp_n[warp] = __popc(bal);
+        if (!__syncthreads_or(bal != 0)) continue;   // nearMat is almost all zeros
+        int before = 0, chunk = 0;
+        for (int w = 0; w < 8; w++) {
+            if (w < warp) before += warp_n[w];
+            chunk += warp_n[w];
+        }
+        if (list && nr) list[base + total + before + __popc(bal & ((1u << lane) - 1u))] = make_int2(t1, t2);
+        total += chunk;
+        __syncthreads();
+    }
+    if (!list && tid == 0) count[t2] = total;
+}
+
+// *asym = 1 when some (t1, t2) is near and (t2, t1) is not
+__global__ void __launch_bounds__(256) k_mat_symmetric(int Nt, const uint8_t *__restrict__ nm, int *__restrict__ asym) {
+    __shared__ uint8_t tile[32][33];
+    if (blockIdx.x > blockIdx.y) return;
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+    for (int j = ty; j < 32; j += 8) {
+        const int r = r0 + tx, c = c0 + j;
+        tile[j][tx] = r < Nt && c < Nt && nm[(size_t)r + (size_t)Nt * c];
+    }
+    __syncthreads();
+    bool bad = false;
+    for (int j = ty; j < 32; j += 8) {   // the transposed tile: row c0 + tx, column r0 + j
+        const int r = c0 + tx, c = r0 + j;
+        if (r < Nt && c < Nt) bad |= (nm[(size_t)r + (size_t)Nt * c] != 0) != (tile[tx][j] != 0);
+    }
+    if (bad) *asym = 1;
+}
+
+// nearMat to the pair mask: 1 = near or self
+__global__ void __launch_bounds__(256) k_mat_mask(int Nt, uint8_t *__restrict__ nm) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (size_t)Nt * Nt) return;
+    nm[i] = nm[i] || i / Nt == i % Nt;
+}
+
 // Exclusive prefix sum of the per-column counts (one CTA); offset[Nt] = total.
 __global__ void __launch_bounds__(1024) k_scan_counts(int Nt, const int *__restrict__ count,
                                                       long long *__restrict__ offset) {
@@ -312,6 +365,42 @@ efie_status efie_geom_precompute_device(efie_ctx *ctx, const efie_mesh *mesh, co
     EFIE_CUDA(cudaGetLastError());
     g.n_near = (int)total;
     g.symmetric = true;
+    EFIE_CUDA(cudaStreamSynchronize(s));   // the temporaries go back to the pool after this
+    return EFIE_OK;
+}
+
+// The near pairs and the pair mask of a host nearMat [Nt x Nt]: the list in
+// column order (t1 < t2 when nearMat is symmetric, else every t1 != t2) and
+// g.symmetric.  nearMat is uploaded into the mask's place; scanning, checking
+// and compacting it on the device leaves the host one copy (Nt 13440, 181 MB).
+efie_status efie_geom_near_device(efie_ctx *ctx, const uint8_t *nearMat, int Nt, GeomDev &g) {
+    cudaStream_t s = ctx->stream;
+    const size_t nn = (size_t)Nt * Nt;
+    EFIE_TRY(g.near_mask.reserve(nn));
+    EFIE_CUDA(cudaMemcpyAsync(g.near_mask.p, nearMat, nn, cudaMemcpyHostToDevice, s));
+    uint8_t *nm = g.near_mask.as<uint8_t>();
+    DevBuf tmp;   // counts [Nt], asym, offsets [Nt + 1]
+    EFIE_TRY(tmp.reserve(sizeof(int) * (Nt + 2) + sizeof(long long) * (Nt + 2)));
+    long long *off = tmp.as<long long>();
+    int *cnt = reinterpret_cast<int *>(off + Nt + 1), *asym = cnt + Nt;
+    EFIE_CUDA(cudaMemsetAsync(asym, 0, sizeof(int), s));
+    const unsigned nb = (Nt + 31) / 32;
+    k_mat_symmetric<<<dim3(nb, nb), 256, 0, s>>>(Nt, nm, asym);
+    k_mat_pairs<<<Nt, 256, 0, s>>>(Nt, nm, asym, cnt, nullptr, nullptr);
+    k_scan_counts<<<1, 1024, 0, s>>>(Nt, cnt, off);
+    EFIE_CUDA(cudaGetLastError());
+    long long total = 0;
+    int bad = 0;
+    EFIE_CUDA(cudaMemcpyAsync(&total, off + Nt, sizeof(long long), cudaMemcpyDeviceToHost, s));
+    EFIE_CUDA(cudaMemcpyAsync(&bad, asym, sizeof(int), cudaMemcpyDeviceToHost, s));
+    EFIE_CUDA(cudaStreamSynchronize(s));
+    if (total > (long long)INT32_MAX) return efie_fail(EFIE_ERR_ARGS, "too many near pairs");
+    EFIE_TRY(g.near_list.reserve(sizeof(int2) * std::max<long long>(total, 1)));
+    if (total > 0) k_mat_pairs<<<Nt, 256, 0, s>>>(Nt, nm, asym, nullptr, off, g.near_list.as<int2>());
+    k_mat_mask<<<(unsigned)((nn + 255) / 256), 256, 0, s>>>(Nt, nm);
+    EFIE_CUDA(cudaGetLastError());
+    g.n_near = (int)total;
+    g.symmetric = bad == 0;
     EFIE_CUDA(cudaStreamSynchronize(s));   // the temporaries go back to the pool after this
     return EFIE_OK;
 }

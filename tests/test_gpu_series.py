@@ -73,6 +73,25 @@ def test_series_z_matches_oracle(name, tiles):
     plan.close()
 
 
+@pytest.mark.parametrize("change", ["half", "off_vertex"])
+def test_series_takes_any_rwg_side(change):
+    """An RWG with one triangle missing, and one whose free vertex is not a vertex of its triangle."""
+    p = eo.build_problem(small_design())
+    r = {k: np.array(v, copy=True) for k, v in p["rwg"].items()}
+    if change == "half":
+        r["minusTri"][5] = 0
+    else:
+        r["rp"][7] += 1e-9 * np.abs(p["V"]).max()
+    p = dict(p, rwg=r)
+    d = p["design"]
+    plan = _plan(p, "ref", 1, d.eps)
+    Z, terms = _series(plan, [2.3e9], 0)
+    omega, k, _, _ = eo.physics(2.3e9, d.mu, d.eps)
+    zo = oc.assemble_z(r, p["prepack"], k, omega, d.mu, d.eps)
+    assert terms > 0 and np.abs(Z[0] - zo).max() < 1e-12 * np.abs(zo).max()
+    plan.close()
+
+
 def test_series_leaves_electrically_large_bases_alone():
     p = eo.build_problem(small_design())
     plan = _plan(p, "ref", 1, eo.EPS0)
