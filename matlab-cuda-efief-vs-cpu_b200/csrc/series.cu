@@ -34,6 +34,7 @@
 
 #include "efie_internal.h"
 #include "quad.cuh"
+#include "warp.cuh"
 
 namespace {
 
@@ -109,103 +110,170 @@ __global__ void __launch_bounds__(128) k_series_reach(int Ne, const int *__restr
 
 // ---------------------------------------------------------------------------
 // Moments of the special triangle pairs about their own base distance Rb
-// (the centroids' distance of a near pair, else 0), eight powers per blockIdx.y:
+// (the centroids' distance of a near pair, else 0):
 // sp[(n * 8 + comp) * nsp + pair], comp = S0, S1xyz (rho, first triangle),
 // S2xyz (rho'), S3 of W t^n / (4 pi R), t = (R - Rb) / delta.  One warp per
-// pair; at 64 accumulators a lane keeps eight powers in registers, and the 64
-// sums are reduced by halving exchanges (each step hands over half of the
-// values still held): 62 exchanges instead of 320.
+// pair.
 // ---------------------------------------------------------------------------
-enum { SP_NEAR = 0, SP_SELF = 1, SP_ADJ = 2 };
+enum { SP_NEAR = 0, SP_SELF = 1 };
 
 struct SpecialArgs {
     int n_pairs, first;          // pairs of this kind, index of the first in the store
     const int2 *list;            // (t1, t2), t1 <= t2 (near, adjacent); self: t = pair index
     int P, per_sub;              // points per triangle, points per sub-triangle (self)
+    int parts;                   // parts of the inner points' loop (near, self)
     const double4 *origin, *pts, *vtx;
     const double *aeq, *self_a;  // softening
     double near_alpha;
     int NsS;
 };
 
-template <int W>
-__device__ __forceinline__ void halve(double (&v)[64], int lane) {
-    constexpr int o = W / 4;   // 64 -> lanes 16 apart, ..., 4 -> lanes 1 apart
-    const bool up = lane & o;
-#pragma unroll
-    for (int i = 0; i < W / 2; i++) {
-        const double keep = up ? v[i + W / 2] : v[i], send = up ? v[i] : v[i + W / 2];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-}
-
-template <int KIND>
-__global__ void __launch_bounds__(64) k_series_special(const SpecialArgs q, double inv_delta, int N, size_t nsp,
-                                                       double *__restrict__ sp) {
+// Near and self pairs, NT powers from NT * blockIdx.y on.  A lane keeps one
+// outer point p (and one of `parts` equal parts of the inner points) at a
+// time: its 4 NT sums of t^n {1, rho'} take five instructions per power and
+// point pair, and the factors 1 and rho_p come in once per outer point, where
+// the eight components are summed over the warp.  Bound by the FP64 pipe:
+// 25 + 5 NT instructions per point pair (eight accumulators per power: 25 + 10
+// per power in chunks of eight, 4.8 ms for 21783 pairs of 96 x 96 points and
+// 14 powers; this form 1.8).
+template <int KIND, int NT>
+__global__ void __launch_bounds__(64) k_series_pairs(const SpecialArgs q, double inv_delta, int N, size_t nsp,
+                                                     double *__restrict__ sp) {
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (w >= q.n_pairs) return;
-    const int n0 = 8 * blockIdx.y;
+    const int n0 = NT * blockIdx.y, P = q.P, items = P * q.parts, len = P / q.parts;
     int2 pr = make_int2(w, w);
-    if (KIND != SP_SELF) pr = q.list[w];
-    const int t1 = pr.x, t2 = pr.y, P = q.P;
+    if (KIND == SP_NEAR) pr = q.list[w];
+    const int t1 = pr.x, t2 = pr.y;
     double dox = 0.0, doy = 0.0, doz = 0.0, a2 = 0.0, Rb = 0.0;
-    if (KIND != SP_SELF) {
+    if (KIND == SP_NEAR) {
         const double4 o1 = q.origin[t1], o2 = q.origin[t2];
         dox = o1.x - o2.x;
         doy = o1.y - o2.y;
         doz = o1.z - o2.z;
-    }
-    if (KIND == SP_NEAR) {
         const double a = q.near_alpha * fmin(q.aeq[t1], q.aeq[t2]);
         a2 = a * a;
         Rb = sqrt(dox * dox + doy * doy + doz * doz);
     }
-    double v[64];
+    constexpr int NG = (NT + 3) / 4;   // groups of four powers: 32 sums, one per lane
+    double sum[NG];
 #pragma unroll
-    for (int i = 0; i < 64; i++) v[i] = 0.0;
+    for (int g = 0; g < NG; g++) sum[g] = 0.0;
+    const double4 *in = q.pts + (size_t)t2 * P;
+#pragma unroll 1
+    for (int it = lane; it - lane < items; it += 32) {
+        double T[NT], X[NT], Y[NT], Z[NT];
+#pragma unroll
+        for (int n = 0; n < NT; n++) T[n] = X[n] = Y[n] = Z[n] = 0.0;
+        double4 pp = make_double4(0, 0, 0, 0);
+        if (it < items) {
+            const int p = it % P, r0 = (it / P) * len;
+            pp = q.pts[(size_t)t1 * P + p];
+            const double px = dox + pp.x, py = doy + pp.y, pz = doz + pp.z, wp = pp.w * (1.0 / (4.0 * kPi));
+            double b2 = 0.0;
+            int s0 = P, s1 = P;   // the inner points of the same sub-triangle
+            if (KIND == SP_SELF) {
+                const int sa = p / q.per_sub;
+                const double aS = q.self_a[(size_t)t1 * q.NsS + sa];
+                b2 = aS * aS;
+                s0 = sa * q.per_sub;
+                s1 = s0 + q.per_sub;
+            }
+#pragma unroll 1
+            for (int r = r0; r < r0 + len; r++) {
+                const double4 pq = in[r];
+                const double dx = px - pq.x, dy = py - pq.y, dz = pz - pq.z;
+                double R2 = dx * dx + dy * dy + dz * dz + (KIND == SP_NEAR ? a2 : 0.0);
+                if (KIND == SP_SELF && r >= s0 && r < s1) R2 += b2;
+                R2 = fmax(R2, 1e-30);
+                const double rs = rsqrt(R2);
+                const double t = (R2 * rs - Rb) * inv_delta;
+                double u = wp * pq.w * rs;
+                for (int i = 0; i < n0; i++) u *= t;
+#pragma unroll
+                for (int n = 0; n < NT; n++) {
+                    T[n] += u;
+                    X[n] = fma(u, pq.x, X[n]);
+                    Y[n] = fma(u, pq.y, Y[n]);
+                    Z[n] = fma(u, pq.z, Z[n]);
+                    u *= t;
+                }
+            }
+        }
+#pragma unroll
+        for (int g = 0; g < NG; g++) {
+            constexpr int last = NT % 4;
+            double d[32];
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                if (4 * g + m >= NT) break;
+                const int n = 4 * g + m;
+                d[8 * m] = T[n];
+                d[8 * m + 1] = T[n] * pp.x;
+                d[8 * m + 2] = T[n] * pp.y;
+                d[8 * m + 3] = T[n] * pp.z;
+                d[8 * m + 4] = X[n];
+                d[8 * m + 5] = Y[n];
+                d[8 * m + 6] = Z[n];
+                d[8 * m + 7] = pp.x * X[n] + pp.y * Y[n] + pp.z * Z[n];
+            }
+            if (last && g == NG - 1) {
+                double h[16];
+#pragma unroll
+                for (int i = 0; i < 16; i++) h[i] = d[i];
+                sum[g] += warp_sums<16>(h, lane);
+            } else {
+                sum[g] += warp_sums<32>(d, lane);
+            }
+        }
+    }
+#pragma unroll
+    for (int g = 0; g < NG; g++) {   // the lane is left with power 4 g + lane / 8, component lane mod 8
+        const int l = 4 * g + (lane >> 3), n = n0 + l;
+        if (l < NT && n < N) sp[((size_t)n * 8 + (lane & 7)) * nsp + q.first + w] = sum[g];
+    }
+}
+
+// Adjacent pairs of the extraction scheme, eight powers per blockIdx.y: the
+// static part (n = 0) is analytic over the inner triangle, the powers from
+// n = 1 on take the rule's point pairs, so few that the lanes share them.
+__global__ void __launch_bounds__(64) k_series_adjacent(const SpecialArgs q, double inv_delta, int N, size_t nsp,
+                                                        double *__restrict__ sp) {
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (w >= q.n_pairs) return;
+    const int n0 = 8 * blockIdx.y, P = q.P;
+    const int2 pr = q.list[w];
+    const int t1 = pr.x, t2 = pr.y;
+    const double4 o1 = q.origin[t1], o2 = q.origin[t2];
+    const double dox = o1.x - o2.x, doy = o1.y - o2.y, doz = o1.z - o2.z;
+    double v[2][32];   // powers n0 .. n0 + 3, n0 + 4 .. n0 + 7
+#pragma unroll
+    for (int i = 0; i < 32; i++) v[0][i] = v[1][i] = 0.0;
     constexpr double k4pi = 1.0 / (4.0 * kPi);
-    const int total = P * P;
-    for (int e = lane; e < total; e += 32) {
+    for (int e = lane; e < P * P; e += 32) {
         const int p = e / P, r = e - p * P;
         const double4 pp = q.pts[(size_t)t1 * P + p], pq = q.pts[(size_t)t2 * P + r];
         const double dx = dox + pp.x - pq.x, dy = doy + pp.y - pq.y, dz = doz + pp.z - pq.z;
-        double R2 = dx * dx + dy * dy + dz * dz + a2;
-        if (KIND == SP_SELF) {
-            const int sa = p / q.per_sub;
-            if (sa == r / q.per_sub) {
-                const double aS = q.self_a[(size_t)t1 * q.NsS + sa];
-                R2 += aS * aS;
-            }
-        }
-        double t, u = pp.w * pq.w * k4pi;
-        double pw = 1.0;   // t^n0 (adjacent pairs: t^(n0 - 1), the static part has n = 0)
-        if (KIND == SP_ADJ) {
-            t = sqrt(R2) * inv_delta;
-            u *= inv_delta;
-        } else {
-            R2 = fmax(R2, 1e-30);
-            const double rs = rsqrt(R2);
-            t = (R2 * rs - Rb) * inv_delta;
-            u *= rs;
-        }
-        for (int i = (KIND == SP_ADJ ? 1 : 0); i < n0; i++) pw *= t;
-        u *= pw;
+        const double t = sqrt(dx * dx + dy * dy + dz * dz) * inv_delta;
+        double u = pp.w * pq.w * k4pi * inv_delta;   // W t^n / (4 pi R) = W t^(n - 1) / (4 pi delta)
+        for (int i = 1; i < n0; i++) u *= t;
         const double dd = pp.x * pq.x + pp.y * pq.y + pp.z * pq.z;
 #pragma unroll
         for (int n = 0; n < 8; n++) {
-            if (KIND == SP_ADJ && n == 0 && n0 == 0) continue;
-            v[8 * n] += u;
-            v[8 * n + 1] += u * pp.x;
-            v[8 * n + 2] += u * pp.y;
-            v[8 * n + 3] += u * pp.z;
-            v[8 * n + 4] += u * pq.x;
-            v[8 * n + 5] += u * pq.y;
-            v[8 * n + 6] += u * pq.z;
-            v[8 * n + 7] += u * dd;
+            if (n == 0 && n0 == 0) continue;
+            double *a = &v[n >> 2][8 * (n & 3)];
+            a[0] += u;
+            a[1] += u * pp.x;
+            a[2] += u * pp.y;
+            a[3] += u * pp.z;
+            a[4] += u * pq.x;
+            a[5] += u * pq.y;
+            a[6] += u * pq.z;
+            a[7] += u * dd;
             u *= t;
         }
     }
-    if (KIND == SP_ADJ && n0 == 0 && lane < P) {
+    if (n0 == 0 && lane < P) {
         // static part: outer point on t1, 1/R integrated analytically over t2
         const double4 pp = q.pts[(size_t)t1 * P + lane];
         const double3 r = make_double3(pp.x + dox, pp.y + doy, pp.z + doz);
@@ -216,25 +284,21 @@ __global__ void __launch_bounds__(64) k_series_special(const SpecialArgs q, doub
                             make_double3(v2.x, v2.y, v2.z), r, I0, J);
         const double sx = J.x + r.x * I0, sy = J.y + r.y * I0, sz = J.z + r.z * I0;
         const double wt = pp.w * k4pi;
-        v[0] += wt * I0;
-        v[1] += wt * I0 * pp.x;
-        v[2] += wt * I0 * pp.y;
-        v[3] += wt * I0 * pp.z;
-        v[4] += wt * sx;
-        v[5] += wt * sy;
-        v[6] += wt * sz;
-        v[7] += wt * (pp.x * sx + pp.y * sy + pp.z * sz);
+        v[0][0] += wt * I0;
+        v[0][1] += wt * I0 * pp.x;
+        v[0][2] += wt * I0 * pp.y;
+        v[0][3] += wt * I0 * pp.z;
+        v[0][4] += wt * sx;
+        v[0][5] += wt * sy;
+        v[0][6] += wt * sz;
+        v[0][7] += wt * (pp.x * sx + pp.y * sy + pp.z * sz);
     }
     __syncwarp();
-    halve<64>(v, lane);
-    halve<32>(v, lane);
-    halve<16>(v, lane);
-    halve<8>(v, lane);
-    halve<4>(v, lane);
 #pragma unroll
-    for (int h = 0; h < 2; h++) {   // the lane is left with sums 2 lane and 2 lane + 1
-        const int i = 2 * lane + h, n = n0 + (i >> 3);
-        if (n < N) sp[((size_t)n * 8 + (i & 7)) * nsp + q.first + w] = v[h];
+    for (int g = 0; g < 2; g++) {
+        const double s = warp_sums<32>(v[g], lane);
+        const int n = n0 + 4 * g + (lane >> 3);
+        if (n < N) sp[((size_t)n * 8 + (lane & 7)) * nsp + q.first + w] = s;
     }
 }
 
@@ -297,11 +361,11 @@ __global__ void __launch_bounds__(128, (N <= 14 ? 4 : 3)) k_series_entries(const
         }
     }
     __syncthreads();
-    const int tx = tid & 31;
+    const int tx = tid & 31, cols = TE / gridDim.y;   // this CTA's columns of the tile
     const int m = bm * TE + tx;
     double *out = mom + (size_t)blockIdx.x * 2 * N * TE * TE + tx;
 #pragma unroll 1
-    for (int j = tid >> 5; j < TE; j += 4) {
+    for (int j = blockIdx.y * cols + (tid >> 5); j < (blockIdx.y + 1) * cols; j += 4) {
         const int n = bn * TE + j;
         const bool on = m < G.Ne && n < G.Ne && !(bm == bn && tx > j);
         double A[N], C[N];
@@ -359,7 +423,9 @@ __global__ void __launch_bounds__(128, (N <= 14 ? 4 : 3)) k_series_entries(const
 // The special pairs' share of the entries: the pair's moments combined for the
 // two basis functions, moved from its base distance to the entry's R0 --
 // int (t + s)^n from int t^n, s = (Rb - R0) / delta, in N - 1 passes
-// M_n += s M_{n-1} -- and added to the entry's sums.
+// M_n += s M_{n-1} -- and added to the entry's sums.  Four CTAs per tile: the
+// tiles along the diagonal hold most of the special pairs, so their columns
+// are spread (127 us with one CTA per tile at Ne 1074).
 // ---------------------------------------------------------------------------
 struct SpecialIndex {
     const int2 *list;   // near or adjacent pairs, ordered by (t2, t1)
@@ -376,8 +442,9 @@ __global__ void __launch_bounds__(256) k_series_add(const SeriesGeom G, int tile
     const int tx = threadIdx.x & 31;
     const int m = bm * TE + tx;
     if (m >= G.Ne) return;
+    const int cols = TE / gridDim.y;
 #pragma unroll 1
-    for (int j = threadIdx.x >> 5; j < TE; j += 8) {
+    for (int j = blockIdx.y * cols + (threadIdx.x >> 5); j < (blockIdx.y + 1) * cols; j += 8) {
         const int n = bn * TE + j;
         if (n >= G.Ne || (bm == bn && tx > j)) continue;
 #pragma unroll 1
@@ -479,8 +546,9 @@ __global__ void __launch_bounds__(256) k_series_eval(int Ne, int tile0, const do
     const int m = bm * TE + tx;
     const bool mirror = bm != bn && bm / 4 == bn / 4;
     const double *in = mom + (size_t)blockIdx.x * 2 * N * TE * TE;
+    const int cols = TE / gridDim.y;
 #pragma unroll 1
-    for (int j = threadIdx.x >> 5; j < TE; j += 8) {
+    for (int j = blockIdx.y * cols + (threadIdx.x >> 5); j < (blockIdx.y + 1) * cols; j += 8) {
         const int n = bn * TE + j;
         if (m >= Ne || n >= Ne) continue;
         // below the diagonal of a diagonal tile: the transposed entry
@@ -609,13 +677,52 @@ size_t special_pairs(const GeomDev &g) {
     return g.scheme == EFIE_SCHEME_EXTRACT ? (size_t)g.n_adj : (size_t)g.n_near + g.Nt;
 }
 
+// CTAs per tile (at most `most`): enough for four per SM where the tiles of a
+// small problem are few
+unsigned tile_split(int tiles, int most) {
+    unsigned y = 1;
+    while ((int)y < most && tiles * (int)y < 600) y *= 2;
+    return y;
+}
+
 template <int NQ, int N>
 efie_status launch_entries(const GeomDev &g, cudaStream_t s, int tile0, int nt, double inv_delta, double *mom) {
     constexpr size_t bytes = sizeof(EntrySmem<NQ>);
     if (bytes > 48 * 1024)
         EFIE_CUDA(cudaFuncSetAttribute(k_series_entries<NQ, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    k_series_entries<NQ, N><<<nt, 128, bytes, s>>>(series_geom(g), tile0, g.reg_pts.as<double4>(), inv_delta, mom);
+    k_series_entries<NQ, N><<<dim3(nt, tile_split(nt, 8)), 128, bytes, s>>>(series_geom(g), tile0, g.reg_pts.as<double4>(), inv_delta, mom);
     return efie_cuda_check(cudaGetLastError(), "series entries");
+}
+
+// Parts of the inner points' loop: the fewest that keep the lanes busiest
+int pair_parts(int P) {
+    int best = 1;
+    double eff = 0.0;
+    for (int parts : {1, 2, 4, 8}) {
+        if (P % parts) continue;
+        const int items = P * parts;
+        const double e = items / (32.0 * ((items + 31) / 32));
+        if (e > eff + 1e-9) eff = e, best = parts;
+    }
+    return best;
+}
+
+template <int KIND>
+efie_status launch_pairs(SpecialArgs q, double inv_delta, int N, size_t nsp, double *sp, cudaStream_t s) {
+    q.parts = pair_parts(q.P);
+    const unsigned nx = (q.n_pairs + 1) / 2;
+    // all powers in one pass up to 16 (4 sums each in registers), else in two
+    switch (N) {
+    case 8: k_series_pairs<KIND, 8><<<nx, 64, 0, s>>>(q, inv_delta, N, nsp, sp); break;
+    case 10: k_series_pairs<KIND, 10><<<nx, 64, 0, s>>>(q, inv_delta, N, nsp, sp); break;
+    case 12: k_series_pairs<KIND, 12><<<nx, 64, 0, s>>>(q, inv_delta, N, nsp, sp); break;
+    case 14: k_series_pairs<KIND, 14><<<nx, 64, 0, s>>>(q, inv_delta, N, nsp, sp); break;
+    case 16: k_series_pairs<KIND, 16><<<nx, 64, 0, s>>>(q, inv_delta, N, nsp, sp); break;
+    case 20: k_series_pairs<KIND, 10><<<dim3(nx, 2), 64, 0, s>>>(q, inv_delta, N, nsp, sp); break;
+    case 24: k_series_pairs<KIND, 12><<<dim3(nx, 2), 64, 0, s>>>(q, inv_delta, N, nsp, sp); break;
+    default: return efie_fail(EFIE_ERR_ARGS, "series: unknown term count");
+    }
+    return efie_cuda_check(cudaGetLastError(), "series pairs");
 }
 
 template <int N>
@@ -632,7 +739,7 @@ efie_status launch_tiles(efie_ctx *ctx, const GeomDev &g, int tile0, int nt, dou
     }
     const bool adj = g.scheme == EFIE_SCHEME_EXTRACT;
     const SpecialIndex X{adj ? g.adj_list.as<int2>() : g.near_list.as<int2>(), adj ? g.n_adj : g.n_near, adj};
-    k_series_add<N><<<nt, 256, 0, s>>>(series_geom(g), tile0, X, special_pairs(g), g.ser_sp.as<double>(), inv, mom);
+    k_series_add<N><<<dim3(nt, 4), 256, 0, s>>>(series_geom(g), tile0, X, special_pairs(g), g.ser_sp.as<double>(), inv, mom);
     EFIE_CUDA(cudaGetLastError());
     // point pairs: four triangle pairs per entry
     ctx->log.end(EFIE_K_QUAD, s, tok, 4.0 * (double)g.Nq * g.Nq * (double)nt * TE * TE, 2);
@@ -648,12 +755,13 @@ efie_status launch_eval(efie_ctx *ctx, const GeomDev &g, int tile0, int nt, cons
     float *pl = po ? po->p : nullptr;
     const size_t ps = po ? po->pstride : 0;
     const int ld = po ? po->ld : 0;
+    const dim3 grid(nt, tile_split(nt, 4));
     size_t tok = ctx->log.begin(s);
     if (lossy)
-        k_series_eval<N, true><<<nt, 256, sm, s>>>(g.Ne, tile0, mom, g.ser_ctr.as<double4>(), nf,
+        k_series_eval<N, true><<<grid, 256, sm, s>>>(g.Ne, tile0, mom, g.ser_ctr.as<double4>(), nf,
                                                    g.ser_coef.as<double>(), even, Zd, zstride, pl, ps, ld);
     else
-        k_series_eval<N, false><<<nt, 256, sm, s>>>(g.Ne, tile0, mom, g.ser_ctr.as<double4>(), nf,
+        k_series_eval<N, false><<<grid, 256, sm, s>>>(g.Ne, tile0, mom, g.ser_ctr.as<double4>(), nf,
                                                     g.ser_coef.as<double>(), even, Zd, zstride, pl, ps, ld);
     EFIE_CUDA(cudaGetLastError());
     // algorithmic bytes: the moments once, Z (and the planes) of every frequency
@@ -740,20 +848,19 @@ efie_status efie_series_begin(efie_ctx *ctx, GeomDev &g, double kabs, double kim
     SpecialArgs q{};
     q.origin = g.origin.as<double4>();
     const double inv = 1.0 / g.ser_delta;
-    const int ny = (N + 7) / 8;
     size_t tok = ctx->log.begin(s);
     int nl = 0;
     double qpe = 0;
     if (ref) {
+        q.n_pairs = g.n_near;
+        q.first = 0;
+        q.list = g.near_list.as<int2>();
+        q.P = g.NsN * g.Nq2;
+        q.pts = g.near_pts.as<double4>();
+        q.aeq = g.aeq.as<double>();
+        q.near_alpha = g.near_alpha;
         if (g.n_near > 0) {
-            q.n_pairs = g.n_near;
-            q.first = 0;
-            q.list = g.near_list.as<int2>();
-            q.P = g.NsN * g.Nq2;
-            q.pts = g.near_pts.as<double4>();
-            q.aeq = g.aeq.as<double>();
-            q.near_alpha = g.near_alpha;
-            k_series_special<SP_NEAR><<<dim3((g.n_near + 1) / 2, ny), 64, 0, s>>>(q, inv, N, nsp, g.ser_sp.as<double>());
+            EFIE_TRY(launch_pairs<SP_NEAR>(q, inv, N, nsp, g.ser_sp.as<double>(), s));
             nl++;
             qpe += (double)q.n_pairs * q.P * q.P;
         }
@@ -764,7 +871,7 @@ efie_status efie_series_begin(efie_ctx *ctx, GeomDev &g, double kabs, double kim
         q.pts = g.self_pts.as<double4>();
         q.self_a = g.self_a.as<double>();
         q.NsS = g.NsS;
-        k_series_special<SP_SELF><<<dim3((g.Nt + 1) / 2, ny), 64, 0, s>>>(q, inv, N, nsp, g.ser_sp.as<double>());
+        EFIE_TRY(launch_pairs<SP_SELF>(q, inv, N, nsp, g.ser_sp.as<double>(), s));
         nl++;
         qpe += (double)q.n_pairs * q.P * q.P;
     } else if (g.n_adj > 0) {
@@ -773,7 +880,7 @@ efie_status efie_series_begin(efie_ctx *ctx, GeomDev &g, double kabs, double kim
         q.P = g.Nq;
         q.pts = g.reg_pts.as<double4>();
         q.vtx = g.tri_vtx.as<double4>();
-        k_series_special<SP_ADJ><<<dim3((g.n_adj + 1) / 2, ny), 64, 0, s>>>(q, inv, N, nsp, g.ser_sp.as<double>());
+        k_series_adjacent<<<dim3((g.n_adj + 1) / 2, (N + 7) / 8), 64, 0, s>>>(q, inv, N, nsp, g.ser_sp.as<double>());
         nl++;
         qpe += (double)q.n_pairs * q.P * (q.P + 1);
     }

@@ -21,6 +21,7 @@
 #include "efie_internal.h"
 #include "solve.h"
 #include "tma.h"
+#include "warp.cuh"
 
 namespace {
 
@@ -181,26 +182,6 @@ struct QrSmem {
     double sum[2 * QC];
     double2 piv[QC];
 };
-
-// sums of n = 32 or 16 values over the warp: lane l is left with value l mod n
-// (each step hands over half of the values still held)
-template <int n>
-__device__ __forceinline__ double warp_sums(double (&d)[n], int lane) {
-    if (n == 16)
-#pragma unroll
-        for (int i = 0; i < n; i++) d[i] += __shfl_xor_sync(0xffffffffu, d[i], 16);
-#pragma unroll
-    for (int o = n / 2; o > 0; o >>= 1) {
-        const bool up = lane & o;
-#pragma unroll
-        for (int i = 0; i < n / 2; i++) {
-            if (i >= o) break;
-            const double keep = up ? d[i + o] : d[i], send = up ? d[i] : d[i + o];
-            d[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-    }
-    return d[0];
-}
 
 // x^H a_c over the warp for the n / 2 columns from c0 on
 template <int n, int QC>
