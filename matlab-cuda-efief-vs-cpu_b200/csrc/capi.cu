@@ -971,9 +971,10 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
         kmax = std::max(kmax, k);
     }
     const int wanted = snapshots_wanted(Nf > 0 ? (kmax - kmin) * p->extent : 0.0);
-    const int na = std::min({Nf, wanted, choose_anchors(N)});
+    // a sweep of no more frequencies than may be factored is one batch
+    const int na = Nf <= choose_anchors(N) ? Nf : std::min(wanted, choose_anchors(N));
     const bool anchored = refines && p->auto_share && p->sw.zsym && p->sw.sym_lu && na <= B;
-    const int lvl1 = anchored && Nf - na > 2 * (wanted - na) ? std::min(B, wanted - na) : 0;
+    const int lvl1 = anchored && na < wanted && Nf - na > 2 * (wanted - na) ? std::min(B, wanted - na) : 0;
     const int tail = anchored ? (Nf - na - lvl1 + B - 1) / B : 0;   // batches of the remaining frequencies
     const int nbat = anchored ? 1 + (lvl1 > 0) + tail : (Nf + B - 1) / B;
     const bool warm = refines && nbat > 1;
@@ -1285,6 +1286,52 @@ extern "C" efie_status efie_patch_sweep_fastquad(efie_ctx *ctx, const efie_mesh 
     return s;
 }
 
+namespace {
+
+// The centroid rule's cache arrays (nearMat null: no near pairs)
+struct CentroidPack {
+    std::vector<double> r, w, a, zero;
+    efie_prepack pre{};
+};
+
+// false where the rule does not fit a prepack: an RWG side whose area is not
+// its triangle's (to rounding), or both sides on one triangle
+bool centroid_pack(const efie_mesh *m, double self_alpha, CentroidPack &c) {
+    const int Nt = m->Nt, Nv = m->Nv;
+    c.r.resize(3 * (size_t)Nt);
+    c.w.resize(Nt);
+    c.a.resize(Nt);
+    c.zero.assign(Nt, 0.0);
+    for (int t = 0; t < Nt; t++) {
+        double r[3][3];
+        for (int j = 0; j < 3; j++)
+            for (int k = 0; k < 3; k++) r[j][k] = m->V[m->F[t + (size_t)j * Nt] - 1 + (size_t)k * Nv];
+        for (int k = 0; k < 3; k++) c.r[3 * (size_t)t + k] = (r[0][k] + r[1][k] + r[2][k]) / 3.0;
+        const double e1[3] = {r[1][0] - r[0][0], r[1][1] - r[0][1], r[1][2] - r[0][2]};
+        const double e2[3] = {r[2][0] - r[0][0], r[2][1] - r[0][1], r[2][2] - r[0][2]};
+        const double cx = e1[1] * e2[2] - e1[2] * e2[1], cy = e1[2] * e2[0] - e1[0] * e2[2],
+                     cz = e1[0] * e2[1] - e1[1] * e2[0];
+        c.w[t] = 0.5 * std::sqrt(cx * cx + cy * cy + cz * cz);
+        c.a[t] = self_alpha * std::sqrt(c.w[t] / 3.141592653589793238462643383279502884);
+    }
+    for (int e = 0; e < m->Ne; e++) {
+        const int tp = m->plusTri[e], tm = m->minusTri[e];
+        if (tp > 0 && tp == tm) return false;
+        if (tp > 0 && !(std::abs(m->Ap[e] - c.w[tp - 1]) <= 1e-14 * c.w[tp - 1])) return false;
+        if (tm > 0 && !(std::abs(m->Am[e] - c.w[tm - 1]) <= 1e-14 * c.w[tm - 1])) return false;
+    }
+    efie_prepack &p = c.pre;
+    p.Nt = Nt;
+    p.Nq = p.Nq2 = p.NsS = p.NsN = 1;
+    p.r_reg = p.self_r = p.near_r = c.r.data();
+    p.w_reg = p.self_w = p.near_w = c.w.data();
+    p.self_a = c.a.data();
+    p.aeqTri = c.zero.data();
+    return true;
+}
+
+}  // namespace
+
 extern "C" efie_status efie_patch_sweep_centroid(efie_ctx *ctx, const efie_mesh *mesh, const double *freqs, int32_t Nf,
                                                  double mu, efie_c128 eps, int32_t patchEdge, int32_t groundEdge,
                                                  double V0, double spreadRadius, double Z0,
@@ -1296,12 +1343,31 @@ extern "C" efie_status efie_patch_sweep_centroid(efie_ctx *ctx, const efie_mesh 
     efie_plan *p = new (std::nothrow) efie_plan();
     if (!p) return efie_fail(EFIE_ERR_NOMEM, "out of host memory");
     p->ctx = ctx;
-    p->centroid = true;
     p->self_alpha = 0.20;  // patch_sweep_cuda.cu:269
     efie_sweep_opts o;
     if (opts) o = *opts;
     else efie_sweep_opts_default(&o);
     o.port_model = EFIE_PORT_EDGE_DIFF;
+    // The one-point rule as a prepack: the centroid with the area as weight,
+    // softened against itself, no near pairs.  Such a sweep runs like any other
+    // (symmetric matrices, L D L^T, series assembly, shared factors): 21 points
+    // of Ne 1074 in 3 ms instead of 6.3.  Areas that are not the triangles' own
+    // keep the assembly that weighs each RWG side by its own area.
+    CentroidPack cp;
+    if (centroid_pack(mesh, p->self_alpha, cp)) {
+        o.scheme = EFIE_SCHEME_REF;
+        if (o.nfreq_hint <= 0) o.nfreq_hint = Nf;
+        efie_status s = plan_common(p, mesh, mu, eps, patchEdge, groundEdge, V0, spreadRadius, Z0, &o);
+        if (s == EFIE_OK) s = efie_geom_upload(ctx, mesh, &cp.pre, EFIE_SCHEME_REF, 0, p->g);
+        if (s == EFIE_OK) {
+            p->sw.zsym = p->g.symmetric;
+            p->sw.planes_from_assembly = p->opts.solver == EFIE_SOLVER_MIXED && p->g.symmetric;
+            s = efie_plan_run(p, freqs, Nf, Zin, S11, I, stats);
+        }
+        efie_plan_destroy(p);
+        return s;
+    }
+    p->centroid = true;
     efie_status s = plan_common(p, mesh, mu, eps, patchEdge, groundEdge, V0, spreadRadius, Z0, &o);
     if (s == EFIE_OK) {
         const int Ne = mesh->Ne, Nt = mesh->Nt, Nv = mesh->Nv;

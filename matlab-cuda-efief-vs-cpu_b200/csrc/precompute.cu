@@ -369,7 +369,7 @@ efie_status efie_geom_precompute_device(efie_ctx *ctx, const efie_mesh *mesh, co
     return EFIE_OK;
 }
 
-// The near pairs and the pair mask of a host nearMat [Nt x Nt]: the list in
+// The near pairs and the pair mask of a host nearMat [Nt x Nt] (null: none): the list in
 // column order (t1 < t2 when nearMat is symmetric, else every t1 != t2) and
 // g.symmetric.  nearMat is uploaded into the mask's place; scanning, checking
 // and compacting it on the device leaves the host one copy (Nt 13440, 181 MB).
@@ -377,8 +377,17 @@ efie_status efie_geom_near_device(efie_ctx *ctx, const uint8_t *nearMat, int Nt,
     cudaStream_t s = ctx->stream;
     const size_t nn = (size_t)Nt * Nt;
     EFIE_TRY(g.near_mask.reserve(nn));
-    EFIE_CUDA(cudaMemcpyAsync(g.near_mask.p, nearMat, nn, cudaMemcpyHostToDevice, s));
     uint8_t *nm = g.near_mask.as<uint8_t>();
+    if (!nearMat) {   // no near pairs
+        EFIE_CUDA(cudaMemsetAsync(nm, 0, nn, s));
+        k_mat_mask<<<(unsigned)((nn + 255) / 256), 256, 0, s>>>(Nt, nm);
+        EFIE_CUDA(cudaGetLastError());
+        EFIE_TRY(g.near_list.reserve(sizeof(int2)));
+        g.n_near = 0;
+        g.symmetric = true;
+        return EFIE_OK;
+    }
+    EFIE_CUDA(cudaMemcpyAsync(nm, nearMat, nn, cudaMemcpyHostToDevice, s));
     DevBuf tmp;   // counts [Nt], asym, offsets [Nt + 1]
     EFIE_TRY(tmp.reserve(sizeof(int) * (Nt + 2) + sizeof(long long) * (Nt + 2)));
     long long *off = tmp.as<long long>();

@@ -43,12 +43,16 @@ static_assert(KMAX == 23, "the wider QR holds 24 columns");
 // three stages: boxes of 8 rows (128 bytes) in the 128-byte swizzle, so that
 // eight lanes on eight rows of one column (as stored) and on eight columns of
 // one row (transposed) both touch eight different 16-byte banks.  Lane
-// (l & 7, l >> 3) of warp w owns y_I[16 w + (l & 7)] and y_I[16 w + 8 + (l & 7)]
-// over every fourth entry; the X slices of the chunk come with it in the stage.
+// (l & 7, l >> 3) of warp w owns y_I[8 w + (l & 7)] over every fourth entry;
+// the X slices of the chunk come with it in the stage.  Ne 6968, 22
+// frequencies, 15 vectors: 7.3 ms, 55 % of the FP64 pipe; eight warps with two
+// rows per lane took 7.9 (two warps per scheduler wait for shared memory), one
+// broadcast entry of X per read with a feeding warp 7.4.
 // ---------------------------------------------------------------------------
 constexpr int MB = 128;                             // rows per item
 constexpr int MC = 32;                              // contraction entries per chunk
 constexpr int MR = 3;                               // stages
+constexpr int MT = 512;                             // threads
 constexpr uint32_t MZ = MB * MC * sizeof(double2);  // 64 KB of Z per chunk
 constexpr uint32_t MX = MC * sizeof(double2);       // one vector's slice
 
@@ -63,7 +67,7 @@ struct SnapIdx {
 };   // a launch takes vectors v0 .. v0 + K - 1 into those columns of W [nf][ldw][N]
 
 template <int K>
-__global__ void __launch_bounds__(256, 1) k_symv_multi(const __grid_constant__ CUtensorMap dmap,
+__global__ void __launch_bounds__(MT, 1) k_symv_multi(const __grid_constant__ CUtensorMap dmap,
                                                        const __grid_constant__ CUtensorMap tmap, int N, int nb, int nf,
                                                        const double2 *__restrict__ xall, const SnapIdx S,
                                                        double2 *__restrict__ W, int v0, int ldw, char *ctl) {
@@ -75,7 +79,7 @@ __global__ void __launch_bounds__(256, 1) k_symv_multi(const __grid_constant__ C
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int G = gridDim.x, items = nb * nf;
     // slices past row N are not copied: what a stage holds there must be finite
-    for (int i = tid; i < MR * K * MC; i += 256)
+    for (int i = tid; i < MR * K * MC; i += MT)
         reinterpret_cast<double2 *>(ring + (i / (K * MC)) * STAGE + MZ)[i % (K * MC)] = make_double2(0.0, 0.0);
     int p_it = blockIdx.x, p_q = 0, issued = 0;   // producer (thread 0): chunk p_q of item p_it is next
     auto produce = [&]() {
@@ -109,36 +113,29 @@ __global__ void __launch_bounds__(256, 1) k_symv_multi(const __grid_constant__ C
     int cc = 0;
     for (int it = blockIdx.x; it < items; it += G) {
         const int f = it / nb, I = it - f * nb;
-        double2 acc[2][K];
+        double2 acc[K];
 #pragma unroll
-        for (int v = 0; v < K; v++) acc[0][v] = acc[1][v] = make_double2(0.0, 0.0);
+        for (int v = 0; v < K; v++) acc[v] = make_double2(0.0, 0.0);
 #pragma unroll 1
         for (int q = 0; q < 4 * nb; q++) {
             if (!mbar_wait_bounded(full + cc % MR, (uint32_t)(cc / MR) & 1u)) fail = 1;
             const unsigned char *st = ring + (cc % MR) * STAGE;
             if (!fail) {
-                const double2 *X = reinterpret_cast<const double2 *>(st + MZ);
-                const bool direct = (q >> 2) >= I;   // block-uniform
-#pragma unroll 1
+                const double2 *X = reinterpret_cast<const double2 *>(st + MZ) + g;
+                // the entry of contraction index 4 c8 + g: box, row and 16-byte
+                // chunk of the swizzle as stored, or transposed (block-uniform)
+                const bool direct = (q >> 2) >= I;
+                const unsigned char *zb = direct ? st + warp * 4096 + g * 128 : st + (8 * warp + li) * 128;
+#pragma unroll 2
                 for (int c8 = 0; c8 < MC / 4; c8++) {
-                    const int c = 4 * c8 + g;
-                    const unsigned char *p0, *p1;
-                    if (direct) {
-                        p0 = st + (2 * warp) * 4096 + c * 128 + ((li ^ (c & 7)) << 4);
-                        p1 = p0 + 4096;
-                    } else {
-                        p0 = st + (c >> 3) * 16384 + (16 * warp + li) * 128 + (((c & 7) ^ li) << 4);
-                        p1 = p0 + 8 * 128;
-                    }
-                    const double2 a0 = *reinterpret_cast<const double2 *>(p0);
-                    const double2 a1 = *reinterpret_cast<const double2 *>(p1);
+                    const int h = (c8 & 1) * 4 + g;   // contraction index mod 8
+                    const unsigned char *p = zb + (direct ? c8 * 512 : (c8 >> 1) * 16384) + ((li ^ h) << 4);
+                    const double2 a = *reinterpret_cast<const double2 *>(p);
 #pragma unroll
                     for (int v = 0; v < K; v++) {
-                        const double2 x = X[v * MC + c];
-                        acc[0][v].x = fma(a0.x, x.x, fma(-a0.y, x.y, acc[0][v].x));
-                        acc[0][v].y = fma(a0.x, x.y, fma(a0.y, x.x, acc[0][v].y));
-                        acc[1][v].x = fma(a1.x, x.x, fma(-a1.y, x.y, acc[1][v].x));
-                        acc[1][v].y = fma(a1.x, x.y, fma(a1.y, x.x, acc[1][v].y));
+                        const double2 x = X[v * MC + 4 * c8];
+                        acc[v].x = fma(a.x, x.x, fma(-a.y, x.y, acc[v].x));
+                        acc[v].y = fma(a.x, x.y, fma(a.y, x.x, acc[v].y));
                     }
                 }
             }
@@ -154,19 +151,17 @@ __global__ void __launch_bounds__(256, 1) k_symv_multi(const __grid_constant__ C
             if (tid == 0) produce();
             cc++;
         }
+        const int m = I * MB + 8 * warp + li;
 #pragma unroll
-        for (int r = 0; r < 2; r++)
+        for (int v = 0; v < K; v++) {
+            double2 s = acc[v];
 #pragma unroll
-            for (int v = 0; v < K; v++) {
-                double2 s = acc[r][v];
-#pragma unroll
-                for (int o = 8; o <= 16; o <<= 1) {
-                    s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-                    s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-                }
-                const int m = I * MB + 16 * warp + 8 * r + li;
-                if (g == (v & 3) && m < N && v0 + v < ldw) W[((size_t)f * ldw + v0 + v) * N + m] = s;
+            for (int o = 8; o <= 16; o <<= 1) {
+                s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+                s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
             }
+            if (g == (v & 3) && m < N && v0 + v < ldw) W[((size_t)f * ldw + v0 + v) * N + m] = s;
+        }
     }
 }
 
@@ -343,7 +338,7 @@ efie_status launch_multi(efie_ctx *ctx, const CUtensorMap &d, const CUtensorMap 
                          const double2 *xall, const SnapIdx &S, double2 *W, int v0, int ldw, char *ctl) {
     const int nb = (N + MB - 1) / MB;
     EFIE_CUDA(cudaFuncSetAttribute(k_symv_multi<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)multi_smem<K>()));
-    k_symv_multi<K><<<std::min(ctx->num_sms, nb * nf), 256, multi_smem<K>(), ctx->stream>>>(d, t, N, nb, nf, xall, S, W,
+    k_symv_multi<K><<<std::min(ctx->num_sms, nb * nf), MT, multi_smem<K>(), ctx->stream>>>(d, t, N, nb, nf, xall, S, W,
                                                                                            v0, ldw, ctl);
     return efie_cuda_check(cudaGetLastError(), "snapshot products");
 }
