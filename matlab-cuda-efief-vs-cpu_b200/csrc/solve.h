@@ -31,7 +31,7 @@ __device__ __forceinline__ float efie_pow2_scale(float mx) {
 struct SolveWork {
     int N = 0, ld = 0, nblk = 0;
     int B = 0;                // batch slots (frequencies solved together)
-    int epoch = 0;            // triangular-solve epoch (tags the progress counters)
+    int epoch = 0;            // triangular-solve epoch (tags the words of solved blocks)
     size_t pstride = 0;       // floats per frequency in `planes` (2 * ld * N)
     size_t dstride = 0;       // float2 per frequency in `dinv`
     int vstride = 0;          // float2 per frequency in each vector of `vec`
@@ -44,7 +44,7 @@ struct SolveWork {
     DevBuf planes;   // per f: float re[N][ld], im[N][ld]  (row-major)
     DevBuf dinv;     // per f: float2 [nblk][2][NB*NB] (L^-1, U^-1 of each diagonal block)
     DevBuf vec;      // float2 rf[B][vstride], y[B][vstride], d[B][vstride]
-    DevBuf prog;     // triangular-solve progress counters: u64 [2][B][grid] on 64-byte lines
+    DevBuf yll;      // solved blocks of a triangular solve: {value, epoch} words u64 [2][B][nblk * 64][2]
     DevBuf ctl;      // per f 64 bytes: red[3] @0, counter @24, conv @28, skip @32, err @36
     DevBuf rpart;    // residual-norm partial sums: double [B][ceil(N/32)]
     DevBuf active;   // int[B]: slot holds a frequency of this batch

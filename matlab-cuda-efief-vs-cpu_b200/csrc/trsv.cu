@@ -6,13 +6,15 @@
 // every dependency of an item sits earlier in some CTA's queue (no deadlock
 // while all CTAs are resident, which the cooperative launch guarantees).
 //
-// Progress is published per (direction, frequency) as a 64-bit counter
-// (epoch << 32 | blocks done) replicated once per CTA on its own 64-byte
-// line: the CTA that finishes a block raises every replica with atomicMax,
-// and a waiting CTA polls only its own replica, so no line is polled by more
-// than one CTA.  Waits are bounded and abort on the frequency's error flag.
-// Nothing a CTA reads from the factors depends on a counter, so its tiles and
-// diagonal inverses stream through a TMA ring ahead of the solve (k_trsv).
+// A solved block is handed on in the words that carry it: each float of y goes
+// out as one 64-bit word {value, epoch}, and a CTA that needs the block reads
+// the words until both epochs of every element are this launch's.  One store
+// and one read through L2 per link of the chain: a separate progress counter
+// costs a fence, an atomic per waiting CTA and a second read.  64-bit accesses
+// are single words of the memory model, so no fence is needed.  Waits are
+// bounded and abort on the frequency's error flag.  Nothing a CTA reads from
+// the factors depends on a solved block, so its tiles and diagonal inverses
+// stream through a TMA ring ahead of the solve (k_trsv).
 #include <algorithm>
 #include <cstdint>
 
@@ -26,34 +28,30 @@ namespace {
 using namespace efie_tma;
 
 constexpr int NB = 64;
-constexpr int LINE = 8;       // u64 per 64-byte progress line
 
 // Limits of the bounded waits, per device.  d_wait_spins: polls before a
-// wait gives up (2^23, about a second).  d_wait_offset: added to every wait
-// target; nonzero only under efie_debug_set_wait_test, where it makes every
-// target unreachable (a count no block ever publishes) so that tests can make
-// the waits run out on purpose.
+// wait gives up (2^23, about a second).  d_wait_offset: added to the epoch a
+// wait looks for; nonzero only under efie_debug_set_wait_test, where it makes
+// every wait look for an epoch that no launch has, so that tests can make the
+// waits run out on purpose.
 __device__ long long d_wait_spins = 1ll << 23;
-__device__ unsigned long long d_wait_offset = 0;
+__device__ unsigned int d_wait_offset = 0;
 
-// Wait until the counter reaches `target`; returns the observed value (0 on
-// timeout or error, after which every waiter returns).
-__device__ __forceinline__ unsigned long long wait_progress(const volatile unsigned long long *ctr,
-                                                            unsigned long long target, const volatile int *err) {
-    long long spins = 0;
-    const long long limit = d_wait_spins;
-    target += d_wait_offset;
-    unsigned long long v;
-    while ((v = *ctr) < target) {
-        if (++spins > limit) {  // give up: record, let every waiter return
-            atomicExch((int *)err, 2);
-            return 0;
-        }
-        if ((spins & 63) == 0 && *err) return 0;
-        __nanosleep(40);
-    }
-    __threadfence();
+__device__ __forceinline__ ulonglong2 ll_load(const ulonglong2 *p) {
+    ulonglong2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
     return v;
+}
+
+__device__ __forceinline__ void ll_store(ulonglong2 *p, float2 y, unsigned int epoch) {
+    const unsigned long long t = (unsigned long long)epoch << 32;
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(t | __float_as_uint(y.x)),
+                 "l"(t | __float_as_uint(y.y))
+                 : "memory");
+}
+
+__device__ __forceinline__ bool ll_ready(const ulonglong2 &v, unsigned int epoch) {
+    return (unsigned int)(v.x >> 32) == epoch && (unsigned int)(v.y >> 32) == epoch;
 }
 
 constexpr int TS = 3;                                          // stages of the tile ring
@@ -94,27 +92,26 @@ __device__ __forceinline__ void stage_row(float4 (&t)[8], const unsigned char *s
 // diagonal inverse (one bulk copy) -- flows through a ring of TS stages fed
 // by thread 0 in the CTA's item order, so the loads of later tiles, and of
 // the next items, are in flight while the CTA waits for a solved block or
-// works on the current one.  The right-hand side blocks y_jb are read from
-// global memory after their publication (one block ahead when already
-// published).
+// works on the current one.  64 threads read a solved block's words, one block
+// ahead of its use, and spread it through shared memory.
 template <bool LOWER>
 __global__ void __launch_bounds__(256, 2) k_trsv(const __grid_constant__ CUtensorMap map, int N, int nblk, int B,
                                                  const float2 *__restrict__ dinv, size_t dstride,
                                                  const float2 *__restrict__ rhsb, float2 *outb, int vstride,
-                                                 double2 *__restrict__ xb, unsigned long long *prog, int epoch,
+                                                 double2 *__restrict__ xb, ulonglong2 *__restrict__ yll, int epoch,
                                                  char *ctl, const int *__restrict__ active,
                                                  const int *__restrict__ fsrc) {
     extern __shared__ unsigned char dsm[];
     __shared__ float2 acc[NB];
     __shared__ float2 part[4][NB];
-    __shared__ int avail_sh, ok, fail;
+    __shared__ float2 ysh[2][NB];
+    __shared__ int ok, fail;
     unsigned char *ring = dsm + (((smem_u32(dsm) + 1023u) & ~1023u) - smem_u32(dsm));
     uint64_t *full = reinterpret_cast<uint64_t *>(ring + TS * STAGE_BYTES);
     const int tid = threadIdx.x;
     const int row = tid & 63, quarter = tid >> 6;
     const int G = gridDim.x;
-    const unsigned long long tag = (unsigned long long)(unsigned)epoch << 32;
-    const int dir = LOWER ? 0 : 1;
+    const unsigned int tag = (unsigned int)epoch, target = tag + d_wait_offset;
     const int items = nblk * B;
     auto live = [&](int it) -> bool {
         const int f = it % B;
@@ -167,7 +164,7 @@ __global__ void __launch_bounds__(256, 2) k_trsv(const __grid_constant__ CUtenso
     // thread 0 drains the pieces in flight before the CTA returns early
     auto drain = [&]() {
         if (tid != 0) return;
-        for (int k = cc; k < issued; k++)
+        for (int k = cc > 0 ? cc - 1 : 0; k < issued; k++)
             if (!mbar_wait_bounded(full + k % TS, (uint32_t)(k / TS) & 1u)) return;
     };
     for (int it = blockIdx.x; it < items; it += G) {
@@ -178,66 +175,54 @@ __global__ void __launch_bounds__(256, 2) k_trsv(const __grid_constant__ CUtenso
         const int b = LOWER ? o : nblk - 1 - o;
         const float2 *rhs = rhsb + (size_t)vstride * f;
         float2 *out = outb + (size_t)vstride * f;
-        unsigned long long *myctr = prog + ((size_t)(dir * B + f) * G + blockIdx.x) * LINE;
+        ulonglong2 *yf = yll + ((size_t)(LOWER ? 0 : B) + f) * nblk * NB;   // this direction's words of f
         const int r0 = b * NB;
         const int rows = min(NB, N - r0);
         if (tid < NB) acc[tid] = (tid < rows) ? rhs[r0 + tid] : make_float2(0.f, 0.f);
-        if (tid == 0) ok = 1, avail_sh = 0;
+        if (tid == 0) ok = 1;
         __syncthreads();
         // each thread keeps its quarter-row dot product in registers across the
-        // dependencies; the CTA synchronises to wait for a block only when the
-        // last observed count does not cover it (one count can cover many)
+        // dependencies
         float2 sdot = make_float2(0.f, 0.f);
-        int avail = 0;
-        float2 ynext[16];
-        bool have_next = false;
-        auto load_y = [&](float2 (&y)[16], int jb) {
-            const float2 *ysrc = out + jb * NB + quarter * 16;
-#pragma unroll
-            for (int k = 0; k < 16; k++) y[k] = (jb * NB + quarter * 16 + k < N) ? ysrc[k] : make_float2(0.f, 0.f);
-        };
+        ulonglong2 w{0, 0};   // the words of the next block (tid < 64), read ahead
+        if (tid < NB && o > 0) w = ll_load(yf + (LOWER ? 0 : nblk - 1) * NB + tid);
         for (int q = 0; q < o; q++) {
             const int jb = LOWER ? q : nblk - 1 - q;
-            if (q >= avail) {
-                if (tid == 0) {
-                    const unsigned long long v = wait_progress(myctr, tag | (unsigned long long)(q + 1), err);
-                    if (!v) ok = 0;
-                    avail_sh = (int)(v & 0xffffffffull);
+            if (tid < NB) {
+                const long long limit = d_wait_spins;
+                for (long long spins = 0; !ll_ready(w, target); w = ll_load(yf + jb * NB + tid)) {
+                    if (++spins > limit) {   // give up: record, let every waiter return
+                        atomicExch((int *)err, 2);
+                        ok = 0;
+                        break;
+                    }
+                    if ((spins & 63) == 0 && *err) {
+                        ok = 0;
+                        break;
+                    }
+                    if (spins > 4) __nanosleep(20);
                 }
-                __syncthreads();
-                if (!ok) {
-                    drain();
-                    return;
-                }
-                avail = avail_sh;
+                ysh[q & 1][tid] = make_float2(__uint_as_float((unsigned int)w.x), __uint_as_float((unsigned int)w.y));
+                if (q + 1 < o) w = ll_load(yf + (LOWER ? jb + 1 : jb - 1) * NB + tid);
             }
-            // block jb of the solution: written by another CTA and published
-            // before `avail` was read, then never changed in this launch
-            float2 y16[16];
-            if (have_next) {
-#pragma unroll
-                for (int k = 0; k < 16; k++) y16[k] = ynext[k];
-            } else {
-                load_y(y16, jb);
-            }
-            have_next = q + 1 < o && q + 1 < avail;
-            if (have_next) load_y(ynext, LOWER ? jb + 1 : jb - 1);
-            const unsigned char *st = take();
-            if (!fail) {
-                float4 t[8];
-                stage_row(t, st, row, quarter);
-                const float2 d = dot16(t, y16);
-                sdot.x += d.x;
-                sdot.y += d.y;
-            }
+            // the block is in shared memory, and every thread is done with the
+            // stage of the block before: it may be refilled
             __syncthreads();
-            if (fail) {
-                if (tid == 0) atomicExch((int *)err, 2);
+            if (!ok || fail) {
+                if (fail && tid == 0) atomicExch((int *)err, 2);
                 drain();
                 return;
             }
-            if (tid == 0) produce();
+            if (q > 0 && tid == 0) produce();
+            const unsigned char *st = take();
             cc++;
+            if (!fail) {
+                float4 t[8];
+                stage_row(t, st, row, quarter);
+                const float2 d = dot16(t, ysh[q & 1] + quarter * 16);
+                sdot.x += d.x;
+                sdot.y += d.y;
+            }
         }
         part[quarter][row] = sdot;
         __syncthreads();
@@ -268,14 +253,25 @@ __global__ void __launch_bounds__(256, 2) k_trsv(const __grid_constant__ CUtenso
             }
             part[quarter][row] = sv;
         }
+        cc++;
         __syncthreads();
         if (fail) {
             if (tid == 0) atomicExch((int *)err, 2);
             drain();
             return;
         }
-        if (tid == 0) produce();
-        cc++;
+        if (tid < NB) {   // the words go out first: the chain waits for them
+            float2 t = make_float2(0.f, 0.f);
+            if (tid < rows) {
+                t.x = part[0][tid].x + part[1][tid].x + part[2][tid].x + part[3][tid].x;
+                t.y = part[0][tid].y + part[1][tid].y + part[2][tid].y + part[3][tid].y;
+            }
+            ll_store(yf + b * NB + tid, t, tag);
+        }
+        if (tid == 0) {
+            if (o > 0) produce();   // the last tile's stage
+            produce();              // the inverse's
+        }
         if (tid < rows) {
             float2 t;
             t.x = part[0][tid].x + part[1][tid].x + part[2][tid].x + part[3][tid].x;
@@ -289,23 +285,18 @@ __global__ void __launch_bounds__(256, 2) k_trsv(const __grid_constant__ CUtenso
                 x[r0 + tid] = xv;
             }
         }
-        __threadfence();
-        __syncthreads();
-        // publish: o + 1 blocks of (dir, f) are done, on every CTA's replica
-        const unsigned long long v = tag | (unsigned long long)(o + 1);
-        unsigned long long *base = prog + (size_t)(dir * B + f) * G * LINE;
-        for (int t = tid; t < G; t += 256) atomicMax(base + (size_t)t * LINE, v);
+        __syncthreads();   // part is free for the next item
     }
 }
 
 }  // namespace
 
 // Test hook (process-wide, on the current device): every later triangular
-// solve waits for a count that is never published and gives up after `spins`
+// solve waits for an epoch that no launch has and gives up after `spins`
 // polls (enable = 1), or the production limits come back (enable = 0).
 extern "C" efie_status efie_debug_set_wait_test(int32_t enable, int64_t spins) {
     const long long lim = enable ? (long long)std::max<int64_t>(spins, 1) : (1ll << 23);
-    const unsigned long long off = enable ? (1ull << 31) : 0ull;   // block counts stay below 2^31
+    const unsigned int off = enable ? 1u << 31 : 0u;   // epochs stay below 2^31
     EFIE_CUDA(cudaMemcpyToSymbol(d_wait_spins, &lim, sizeof(lim)));
     EFIE_CUDA(cudaMemcpyToSymbol(d_wait_offset, &off, sizeof(off)));
     EFIE_CUDA(cudaDeviceSynchronize());
@@ -323,10 +314,11 @@ efie_status efie_trsv_workspace(SolveWork &w) {
     EFIE_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, k_trsv<false>, 256, TRSV_SMEM));
     occ = std::max(1, std::min(std::min(occ, occ2), 2));
     w.grid = std::max(1, std::min(w.nblk * w.B, occ * sms));
-    const size_t bytes = sizeof(unsigned long long) * LINE * 2 * (size_t)w.B * w.grid;
-    if (bytes > w.prog.bytes) {
-        EFIE_TRY(w.prog.reserve(bytes));
-        EFIE_CUDA(cudaMemset(w.prog.p, 0, bytes));  // epoch 0 < every real epoch
+    const size_t bytes = sizeof(ulonglong2) * 2 * (size_t)w.B * w.nblk * NB;
+    if (bytes > w.yll.bytes) {
+        EFIE_TRY(w.yll.reserve(bytes));
+        EFIE_CUDA(cudaMemset(w.yll.p, 0, w.yll.bytes));  // epoch 0 < every real epoch
+        w.epoch = 0;
     }
     return EFIE_OK;
 }
@@ -337,13 +329,13 @@ efie_status efie_trsv(efie_ctx *ctx, SolveWork &w, bool lower, const float2 *rhs
     int grid = w.grid;
     const float2 *dinv = w.dinv.as<float2>();
     double2 *xd = static_cast<double2 *>(x);
-    unsigned long long *prog = w.prog.as<unsigned long long>();
+    ulonglong2 *yll = w.yll.as<ulonglong2>();
     char *ctl = w.ctl.as<char>();
     const int *active = w.active.as<int>();
     const int *fsrc = w.fsrc_on ? w.fsrc.as<int>() : nullptr;
     void *args[] = {(void *)w.planes_map, (void *)&w.N,   (void *)&w.nblk,    (void *)&w.B,  (void *)&dinv,
                     (void *)&w.dstride,   (void *)&rhs,   (void *)&out,       (void *)&w.vstride,
-                    (void *)&xd,          (void *)&prog,  (void *)&epoch,     (void *)&ctl,  (void *)&active,
+                    (void *)&xd,          (void *)&yll,  (void *)&epoch,     (void *)&ctl,  (void *)&active,
                     (void *)&fsrc};
     const void *fn = lower ? (const void *)k_trsv<true> : (const void *)k_trsv<false>;
     EFIE_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(256), args, TRSV_SMEM, ctx->stream));
