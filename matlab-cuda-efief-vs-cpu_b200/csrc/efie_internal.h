@@ -181,9 +181,9 @@ struct GeomDev {
     int n_reg_tiles = 0;
     // series assembly (series.cu): RWG centres, half-width of R - R0 (0 until
     // the first sweep measures it), coefficients of a batch, special pairs'
-    // moments, and the moments of the entries in `moments` (ser_cap of the
+    // moments, whether a tile holds any, and the entries' moments in `moments` (ser_cap of the
     // ser_tiles tiles at a time; ser_done: all of this sweep's are there)
-    DevBuf ser_ctr, ser_coef, ser_sp;
+    DevBuf ser_ctr, ser_coef, ser_sp, ser_flag;
     double ser_delta = 0.0;
     int ser_n = 0;            // terms of the current sweep
     size_t ser_cap = 0, ser_tiles = 0;

@@ -323,7 +323,8 @@ template <int NQ, int N>
 __global__ void __launch_bounds__(128, (N <= 14 ? 4 : 3)) k_series_entries(const SeriesGeom G, int tile0,
                                                                           const double4 *__restrict__ pts,
                                                                           double inv_delta,
-                                                                          double *__restrict__ mom) {
+                                                                          double *__restrict__ mom,
+                                                                          int *__restrict__ special) {
     extern __shared__ __align__(16) unsigned char raw[];
     EntrySmem<NQ> &S = *reinterpret_cast<EntrySmem<NQ> *>(raw);
     int bm, bn;
@@ -364,6 +365,7 @@ __global__ void __launch_bounds__(128, (N <= 14 ? 4 : 3)) k_series_entries(const
     const int tx = tid & 31, cols = TE / gridDim.y;   // this CTA's columns of the tile
     const int m = bm * TE + tx;
     double *out = mom + (size_t)blockIdx.x * 2 * N * TE * TE + tx;
+    bool any = false;   // a special pair among this CTA's entries
 #pragma unroll 1
     for (int j = blockIdx.y * cols + (tid >> 5); j < (blockIdx.y + 1) * cols; j += 4) {
         const int n = bn * TE + j;
@@ -379,7 +381,11 @@ __global__ void __launch_bounds__(128, (N <= 14 ? 4 : 3)) k_series_entries(const
             const int a = ab >> 1, b = ab & 1;
             const int t1 = S.t[0][a][tx], t2 = S.t[1][b][j];
             if (t2 < 0) continue;
-            if (!on || t1 < 0 || G.mask[(size_t)t1 + (size_t)G.Nt * t2]) continue;
+            if (!on || t1 < 0) continue;
+            if (G.mask[(size_t)t1 + (size_t)G.Nt * t2]) {
+                any = true;
+                continue;
+            }
             const double ox = S.o[0][3 * a][tx] - S.o[1][3 * b][j], oy = S.o[0][3 * a + 1][tx] - S.o[1][3 * b + 1][j],
                          oz = S.o[0][3 * a + 2][tx] - S.o[1][3 * b + 2][j];
 #pragma unroll 1
@@ -417,6 +423,8 @@ __global__ void __launch_bounds__(128, (N <= 14 ? 4 : 3)) k_series_entries(const
             out[(size_t)(N + i) * TE * TE + j * TE] = C[i];
         }
     }
+    any = __syncthreads_or(any);
+    if (tid == 0) special[blockIdx.x * gridDim.y + blockIdx.y] = any;
 }
 
 // ---------------------------------------------------------------------------
@@ -436,7 +444,12 @@ struct SpecialIndex {
 template <int N>
 __global__ void __launch_bounds__(256) k_series_add(const SeriesGeom G, int tile0, const SpecialIndex X, size_t nsp,
                                                     const double *__restrict__ sp, double inv_delta,
-                                                    double *__restrict__ mom) {
+                                                    double *__restrict__ mom, const int *__restrict__ special,
+                                                    int split) {
+    // most tiles hold no special pair: k_series_entries has seen every one
+    bool any = false;
+    for (int i = 0; i < split; i++) any |= special[blockIdx.x * split + i] != 0;
+    if (!any) return;
     int bm, bn;
     tri_tile(tile0 + blockIdx.x, bm, bn);
     const int tx = threadIdx.x & 31;
@@ -686,11 +699,13 @@ unsigned tile_split(int tiles, int most) {
 }
 
 template <int NQ, int N>
-efie_status launch_entries(const GeomDev &g, cudaStream_t s, int tile0, int nt, double inv_delta, double *mom) {
+efie_status launch_entries(const GeomDev &g, cudaStream_t s, int tile0, int nt, double inv_delta, double *mom,
+                           int *special) {
     constexpr size_t bytes = sizeof(EntrySmem<NQ>);
     if (bytes > 48 * 1024)
         EFIE_CUDA(cudaFuncSetAttribute(k_series_entries<NQ, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    k_series_entries<NQ, N><<<dim3(nt, tile_split(nt, 8)), 128, bytes, s>>>(series_geom(g), tile0, g.reg_pts.as<double4>(), inv_delta, mom);
+    k_series_entries<NQ, N><<<dim3(nt, tile_split(nt, 8)), 128, bytes, s>>>(series_geom(g), tile0, g.reg_pts.as<double4>(), inv_delta, mom,
+                                                                                      special);
     return efie_cuda_check(cudaGetLastError(), "series entries");
 }
 
@@ -729,17 +744,19 @@ template <int N>
 efie_status launch_tiles(efie_ctx *ctx, const GeomDev &g, int tile0, int nt, double *mom) {
     cudaStream_t s = ctx->stream;
     const double inv = 1.0 / g.ser_delta;
+    int *flags = g.ser_flag.as<int>();
     size_t tok = ctx->log.begin(s);
     switch (g.Nq) {
-    case 1: EFIE_TRY((launch_entries<1, N>(g, s, tile0, nt, inv, mom))); break;
-    case 3: EFIE_TRY((launch_entries<3, N>(g, s, tile0, nt, inv, mom))); break;
-    case 6: EFIE_TRY((launch_entries<6, N>(g, s, tile0, nt, inv, mom))); break;
-    case 7: EFIE_TRY((launch_entries<7, N>(g, s, tile0, nt, inv, mom))); break;
+    case 1: EFIE_TRY((launch_entries<1, N>(g, s, tile0, nt, inv, mom, flags))); break;
+    case 3: EFIE_TRY((launch_entries<3, N>(g, s, tile0, nt, inv, mom, flags))); break;
+    case 6: EFIE_TRY((launch_entries<6, N>(g, s, tile0, nt, inv, mom, flags))); break;
+    case 7: EFIE_TRY((launch_entries<7, N>(g, s, tile0, nt, inv, mom, flags))); break;
     default: return efie_fail(EFIE_ERR_ARGS, "series: unsupported rule");
     }
     const bool adj = g.scheme == EFIE_SCHEME_EXTRACT;
     const SpecialIndex X{adj ? g.adj_list.as<int2>() : g.near_list.as<int2>(), adj ? g.n_adj : g.n_near, adj};
-    k_series_add<N><<<dim3(nt, 4), 256, 0, s>>>(series_geom(g), tile0, X, special_pairs(g), g.ser_sp.as<double>(), inv, mom);
+    k_series_add<N><<<dim3(nt, 4), 256, 0, s>>>(series_geom(g), tile0, X, special_pairs(g), g.ser_sp.as<double>(), inv, mom,
+                                              flags, (int)tile_split(nt, 8));
     EFIE_CUDA(cudaGetLastError());
     // point pairs: four triangle pairs per entry
     ctx->log.end(EFIE_K_QUAD, s, tok, 4.0 * (double)g.Nq * g.Nq * (double)nt * TE * TE, 2);
@@ -840,7 +857,9 @@ efie_status efie_series_begin(efie_ctx *ctx, GeomDev &g, double kabs, double kim
     const size_t cap = g.moments.bytes / per;
     if (cap < 1) return EFIE_OK;
     const size_t nsp = special_pairs(g);   // the special pairs' moments
-    if (g.ser_sp.reserve(sizeof(double) * 8 * N * std::max<size_t>(nsp, 1)) != EFIE_OK) return EFIE_OK;
+    if (g.ser_sp.reserve(sizeof(double) * 8 * N * std::max<size_t>(nsp, 1)) != EFIE_OK ||
+        g.ser_flag.reserve(sizeof(int) * 8 * std::min(cap, tiles)) != EFIE_OK)
+        return EFIE_OK;
     g.ser_n = N;
     g.ser_cap = std::min(cap, tiles);
     g.ser_tiles = tiles;

@@ -29,7 +29,8 @@
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16;
+constexpr int BM = 32, BN = 32, BK = 32;
+constexpr int GT = 128;   // threads of a product's CTA
 
 enum Epilogue { EPI_FWD_HIDDEN = 0, EPI_FWD_OUT = 1, EPI_BWD_DZ = 2, EPI_PARTIAL = 3 };
 constexpr int KSPLIT = 512;   // K chunk of the weight-gradient products
@@ -44,64 +45,74 @@ template <>
 __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 
 // C[i][j] (M x N, row stride ldc) = sum_k A(i,k) B(k,j) with A(i,k) =
-// A[i*sai + k*sak] (FP32) and B(k,j) = B[k*sbk + j*sbj]; 64x64 tiles, 4x4
-// outputs per thread, FP32 accumulation.  blockIdx.z splits K in chunks of
+// A[i*sai + k*sak] (FP32) and B(k,j) = B[k*sbk + j*sbj]; FP32 accumulation,
+// one fmaf per k in ascending order.  blockIdx.z splits K in chunks of
 // kchunk; EPI_PARTIAL stores chunk z's partial product at C + z M ldc, and
 // k_sum_parts adds the chunks in order (bit-reproducible gradients).
+//
+// The layers are small (1024 x 256 x 256), so a product is bound by latency:
+// 32 x 32 tiles fill the GPU (256 CTAs for a layer; 64 x 64 tiles left half of
+// the SMs idle), and the next 32 of K are read into registers while the
+// current ones are used.  A training step of five layers of batch 1024 took
+// 480 us with 64 x 64 tiles read between two barriers per 16 of K.
 template <typename TB, int EPI>
-__global__ void __launch_bounds__(256) k_mlp_gemm(int M, int N, int K, const float *__restrict__ A, long sai,
-                                                  long sak, const TB *__restrict__ B, long sbk, long sbj,
-                                                  float *__restrict__ C, int ldc, const float *__restrict__ bias,
-                                                  float *__restrict__ Aout, const float *__restrict__ Zprev,
-                                                  int kchunk) {
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Bs[BK][BN + 4];
+__global__ void __launch_bounds__(GT) k_mlp_gemm(int M, int N, int K, const float *__restrict__ A, long sai,
+                                                 long sak, const TB *__restrict__ B, long sbk, long sbj,
+                                                 float *__restrict__ C, int ldc, const float *__restrict__ bias,
+                                                 float *__restrict__ Aout, const float *__restrict__ Zprev,
+                                                 int kchunk) {
+    __shared__ __align__(16) float As[BK][BM + 4];
+    __shared__ __align__(16) float Bs[BK][BN + 4];
     const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;
+    const int tx = tid & 15, ty = tid >> 4;   // rows 4 ty .., columns 2 tx ..
     const int i0 = blockIdx.y * BM, j0 = blockIdx.x * BN;
     const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
-    float acc[4][4];
+    constexpr int PT = BM * BK / GT;   // elements of each tile per thread
+    const bool ak = sak == 1, bj = sbj == 1;   // contiguous along k, along j
+    float ra[PT], rb[PT];
+    auto fetch = [&](int k0) {
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+        for (int r = 0; r < PT; r++) {
+            const int e = tid + GT * r, hi = e / 32, lo = e % 32;
+            const int gi = i0 + (ak ? hi : lo), gk = k0 + (ak ? lo : hi);
+            ra[r] = (gi < M && gk < kend) ? A[(long)gi * sai + (long)gk * sak] : 0.f;
+            const int gj = j0 + (bj ? lo : hi), gkb = k0 + (bj ? hi : lo);
+            rb[r] = (gj < N && gkb < kend) ? to_f<TB>(B[(long)gkb * sbk + (long)gj * sbj]) : 0.f;
+        }
+    };
+    float acc[4][2];
 #pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = 0.f;
+    for (int a = 0; a < 4; a++) acc[a][0] = acc[a][1] = 0.f;
+    if (kbeg < kend) fetch(kbeg);
     for (int k0 = kbeg; k0 < kend; k0 += BK) {
-        // A tile: BM x BK; B tile: BK x BN (4 elements per thread each)
+        __syncthreads();   // the tiles in shared memory are used up
 #pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int e = tid + 256 * r;
-            int ii, kk;
-            if (sak == 1) { ii = e / BK; kk = e % BK; }   // contiguous along k
-            else { ii = e % BM; kk = e / BM; }            // contiguous along i
-            const int gi = i0 + ii, gk = k0 + kk;
-            As[kk][ii] = (gi < M && gk < kend) ? A[(long)gi * sai + (long)gk * sak] : 0.f;
-            int jj, kb;
-            if (sbj == 1) { jj = e % BN; kb = e / BN; }
-            else { jj = e / BK; kb = e % BK; }
-            const int gj = j0 + jj, gkb = k0 + kb;
-            Bs[kb][jj] = (gj < N && gkb < kend) ? to_f<TB>(B[(long)gkb * sbk + (long)gj * sbj]) : 0.f;
+        for (int r = 0; r < PT; r++) {
+            const int e = tid + GT * r, hi = e / 32, lo = e % 32;
+            As[ak ? lo : hi][ak ? hi : lo] = ra[r];
+            Bs[bj ? hi : lo][bj ? lo : hi] = rb[r];
         }
         __syncthreads();
+        if (k0 + BK < kend) fetch(k0 + BK);
 #pragma unroll
         for (int kk = 0; kk < BK; kk++) {
-            float x[4], y[4];
-#pragma unroll
-            for (int a = 0; a < 4; a++) {
-                x[a] = As[kk][ty * 4 + a];
-                y[a] = Bs[kk][tx * 4 + a];
-            }
-#pragma unroll
-            for (int a = 0; a < 4; a++)
-#pragma unroll
-                for (int b = 0; b < 4; b++) acc[a][b] = fmaf(x[a], y[b], acc[a][b]);
+            const float4 x = *reinterpret_cast<const float4 *>(&As[kk][4 * ty]);
+            const float2 y = *reinterpret_cast<const float2 *>(&Bs[kk][2 * tx]);
+            acc[0][0] = fmaf(x.x, y.x, acc[0][0]);
+            acc[0][1] = fmaf(x.x, y.y, acc[0][1]);
+            acc[1][0] = fmaf(x.y, y.x, acc[1][0]);
+            acc[1][1] = fmaf(x.y, y.y, acc[1][1]);
+            acc[2][0] = fmaf(x.z, y.x, acc[2][0]);
+            acc[2][1] = fmaf(x.z, y.y, acc[2][1]);
+            acc[3][0] = fmaf(x.w, y.x, acc[3][0]);
+            acc[3][1] = fmaf(x.w, y.y, acc[3][1]);
         }
-        __syncthreads();
     }
 #pragma unroll
     for (int a = 0; a < 4; a++)
 #pragma unroll
-        for (int b = 0; b < 4; b++) {
-            const int i = i0 + ty * 4 + a, j = j0 + tx * 4 + b;
+        for (int b = 0; b < 2; b++) {
+            const int i = i0 + ty * 4 + a, j = j0 + tx * 2 + b;
             if (i >= M || j >= N) continue;
             const long o = (long)i * ldc + j;
             if (EPI == EPI_FWD_HIDDEN) {
@@ -136,6 +147,7 @@ __global__ void __launch_bounds__(256) k_colsum(int M, int N, const float *__res
     __shared__ float part[8][33];
     float s = 0.f;
     if (j < N)
+#pragma unroll 16
         for (int i = r; i < M; i += 8) s += dZ[(long)i * N + j];
     part[r][threadIdx.x & 31] = s;
     __syncthreads();
@@ -230,7 +242,11 @@ struct efie_mlp {
     size_t np = 0;
     DevBuf w, wb, g, m, v;                       // params FP32, BF16 copy, grads, Adam moments
     DevBuf act;                                  // Z and A of every layer for `cap` rows
-    DevBuf dz0, dz1;                             // backward ping-pong
+    DevBuf dz;                                   // dZ of every hidden layer
+    // the weight gradients run beside the chain of dZ (fork and join by events,
+    // also inside the captured step)
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_dz = nullptr, ev_side = nullptr;
     DevBuf gpart;                                // K-split partials of the weight gradients
     DevBuf Xd, Td, perm, Xb, Tb, dY, step, hist, loss;
     DevBuf Xin;                                  // inference input
@@ -245,12 +261,15 @@ struct efie_mlp {
     float *A(int l) { return act.as<float>() + (size_t)cap * width * (2 * l + 1); }
     float *Y() { return Z(nl - 1); }
     std::vector<void *> step_ptrs() const {
-        return {w.p,  wb.p, g.p,  m.p,  v.p,  act.p, dz0.p, dz1.p, gpart.p,
+        return {w.p,  wb.p, g.p,  m.p,  v.p,  act.p, dz.p, gpart.p,
                 Xd.p, Td.p, perm.p, Xb.p, Tb.p, dY.p, step.p, hist.p};
     }
 
     ~efie_mlp() {
         if (graph) cudaGraphExecDestroy(graph);
+        if (side) cudaStreamDestroy(side);
+        for (cudaEvent_t e : {ev_dz, ev_side})
+            if (e) cudaEventDestroy(e);
     }
 };
 
@@ -260,8 +279,12 @@ efie_status mlp_reserve(efie_mlp *p, int rows) {
     if (rows <= p->cap) return EFIE_OK;
     const int width = p->width;
     EFIE_TRY(p->act.reserve(sizeof(float) * (size_t)rows * width * 2 * p->nl));
-    EFIE_TRY(p->dz0.reserve(sizeof(float) * (size_t)rows * width));
-    EFIE_TRY(p->dz1.reserve(sizeof(float) * (size_t)rows * width));
+    EFIE_TRY(p->dz.reserve(sizeof(float) * (size_t)rows * width * p->nl));
+    if (!p->side) {
+        EFIE_CUDA(cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking));
+        for (cudaEvent_t *e : {&p->ev_dz, &p->ev_side})
+            EFIE_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    }
     size_t wmax = 0;
     for (int l = 0; l < p->nl; l++) wmax = std::max(wmax, (size_t)p->fin[l] * p->fout[l]);
     EFIE_TRY(p->gpart.reserve(sizeof(float) * wmax * (size_t)cdiv(rows, KSPLIT)));
@@ -284,10 +307,10 @@ efie_status mlp_forward(efie_mlp *p, const float *X, int n) {
         const float *b = p->w.as<float>() + p->boff[l];
         // B(k, j) = W[j][k]
         if (l + 1 < p->nl)
-            k_mlp_gemm<__nv_bfloat16, EPI_FWD_HIDDEN><<<grid, 256, 0, s>>>(n, fo, fi, in, fi, 1, W, 1, fi, p->Z(l), fo, b,
+            k_mlp_gemm<__nv_bfloat16, EPI_FWD_HIDDEN><<<grid, GT, 0, s>>>(n, fo, fi, in, fi, 1, W, 1, fi, p->Z(l), fo, b,
                                                                           p->A(l), nullptr, fi);
         else
-            k_mlp_gemm<__nv_bfloat16, EPI_FWD_OUT><<<grid, 256, 0, s>>>(n, fo, fi, in, fi, 1, W, 1, fi, p->Z(l), fo, b,
+            k_mlp_gemm<__nv_bfloat16, EPI_FWD_OUT><<<grid, GT, 0, s>>>(n, fo, fi, in, fi, 1, W, 1, fi, p->Z(l), fo, b,
                                                                        nullptr, nullptr, fi);
         EFIE_CUDA(cudaGetLastError());
         in = p->A(l);
@@ -301,32 +324,33 @@ efie_status mlp_backward(efie_mlp *p, const float *X, const float *dY, int n) {
     cudaStream_t s = p->ctx->stream;
     const int kchunk = KSPLIT;
     const float *dz = dY;
-    float *bufs[2] = {p->dz0.as<float>(), p->dz1.as<float>()};
-    int pb = 0;
     for (int l = p->nl - 1; l >= 0; l--) {
         const int fi = p->fin[l], fo = p->fout[l];
         const float *ain = l > 0 ? p->A(l - 1) : X;
         float *gW = p->g.as<float>() + p->woff[l], *gb = p->g.as<float>() + p->boff[l];
         // dW[o][i] += sum_m dz[m][o] ain[m][i]:  A(i=o, k=m) = dz[m*fo + o], B(k=m, j=i) = ain[m*fi + i]
+        EFIE_CUDA(cudaEventRecord(p->ev_dz, s));
+        EFIE_CUDA(cudaStreamWaitEvent(p->side, p->ev_dz, 0));
         dim3 gw(cdiv(fi, BN), cdiv(fo, BM), cdiv(n, kchunk));
-        k_mlp_gemm<float, EPI_PARTIAL><<<gw, 256, 0, s>>>(fo, fi, n, dz, 1, fo, ain, fi, 1, p->gpart.as<float>(), fi,
-                                                         nullptr, nullptr, nullptr, kchunk);
+        k_mlp_gemm<float, EPI_PARTIAL><<<gw, GT, 0, p->side>>>(fo, fi, n, dz, 1, fo, ain, fi, 1, p->gpart.as<float>(),
+                                                              fi, nullptr, nullptr, nullptr, kchunk);
         const long cnt = (long)fo * fi;
-        k_sum_parts<<<(unsigned)((cnt + 255) / 256), 256, 0, s>>>((int)gw.z, cnt, p->gpart.as<float>(), gW);
-        k_colsum<<<dim3(cdiv(fo, 32), 1), 256, 0, s>>>(n, fo, dz, gb);
+        k_sum_parts<<<(unsigned)((cnt + 255) / 256), 256, 0, p->side>>>((int)gw.z, cnt, p->gpart.as<float>(), gW);
+        k_colsum<<<dim3(cdiv(fo, 32), 1), 256, 0, p->side>>>(n, fo, dz, gb);
         EFIE_CUDA(cudaGetLastError());
         if (l > 0) {
             // dZ_{l-1}[m][i] = (sum_o dz[m][o] W[o][i]) * silu'(Z_{l-1}[m][i])
-            float *out = bufs[pb];
-            pb ^= 1;
+            float *out = p->dz.as<float>() + (size_t)p->cap * p->width * l;
             const __nv_bfloat16 *W = p->wb.as<__nv_bfloat16>() + p->woff[l];
             dim3 gd(cdiv(fi, BN), cdiv(n, BM), 1);
-            k_mlp_gemm<__nv_bfloat16, EPI_BWD_DZ><<<gd, 256, 0, s>>>(n, fi, fo, dz, fo, 1, W, fi, 1, out, fi, nullptr,
+            k_mlp_gemm<__nv_bfloat16, EPI_BWD_DZ><<<gd, GT, 0, s>>>(n, fi, fo, dz, fo, 1, W, fi, 1, out, fi, nullptr,
                                                                     nullptr, p->Z(l - 1), fo);
             EFIE_CUDA(cudaGetLastError());
             dz = out;
         }
     }
+    EFIE_CUDA(cudaEventRecord(p->ev_side, p->side));
+    EFIE_CUDA(cudaStreamWaitEvent(s, p->ev_side, 0));
     return EFIE_OK;
 }
 
