@@ -30,7 +30,7 @@
 namespace {
 
 constexpr int BM = 32, BN = 32, BK = 32;
-constexpr int GT = 128;   // threads of a product's CTA
+constexpr int GT = 256;   // threads of a product's CTA, 2 x 2 outputs each
 
 enum Epilogue { EPI_FWD_HIDDEN = 0, EPI_FWD_OUT = 1, EPI_BWD_DZ = 2, EPI_PARTIAL = 3 };
 constexpr int KSPLIT = 512;   // K chunk of the weight-gradient products
@@ -61,58 +61,58 @@ __global__ void __launch_bounds__(GT) k_mlp_gemm(int M, int N, int K, const floa
                                                  float *__restrict__ C, int ldc, const float *__restrict__ bias,
                                                  float *__restrict__ Aout, const float *__restrict__ Zprev,
                                                  int kchunk) {
-    __shared__ __align__(16) float As[BK][BM + 4];
-    __shared__ __align__(16) float Bs[BK][BN + 4];
+    __shared__ __align__(8) float As[BK][BM + 2];
+    __shared__ __align__(8) float Bs[BK][BN + 2];
     const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;   // rows 4 ty .., columns 2 tx ..
+    const int tx = tid & 15, ty = tid >> 4;   // rows 2 ty, 2 ty + 1, columns 2 tx, 2 tx + 1
     const int i0 = blockIdx.y * BM, j0 = blockIdx.x * BN;
     const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
-    constexpr int PT = BM * BK / GT;   // elements of each tile per thread
-    const bool ak = sak == 1, bj = sbj == 1;   // contiguous along k, along j
+    constexpr int PT = BM * BK / GT, PS = GT / 32;   // elements of each tile per thread, their stride
+    const bool ak = sak == 1, bj = sbj == 1;         // contiguous along k, along j
+    const int hi = tid >> 5, lo = tid & 31;
+    const float *pa = A + (long)(i0 + (ak ? hi : lo)) * sai + (long)(kbeg + (ak ? lo : hi)) * sak;
+    const TB *pb = B + (long)(kbeg + (bj ? hi : lo)) * sbk + (long)(j0 + (bj ? lo : hi)) * sbj;
+    const long da = PS * (ak ? sai : sak), db = PS * (bj ? sbk : sbj), na = BK * sak, nb = BK * sbk;
     float ra[PT], rb[PT];
     auto fetch = [&](int k0) {
 #pragma unroll
         for (int r = 0; r < PT; r++) {
-            const int e = tid + GT * r, hi = e / 32, lo = e % 32;
-            const int gi = i0 + (ak ? hi : lo), gk = k0 + (ak ? lo : hi);
-            ra[r] = (gi < M && gk < kend) ? A[(long)gi * sai + (long)gk * sak] : 0.f;
-            const int gj = j0 + (bj ? lo : hi), gkb = k0 + (bj ? hi : lo);
-            rb[r] = (gj < N && gkb < kend) ? to_f<TB>(B[(long)gkb * sbk + (long)gj * sbj]) : 0.f;
+            const int h = hi + PS * r;
+            const bool oa = ak ? i0 + h < M && k0 + lo < kend : i0 + lo < M && k0 + h < kend;
+            const bool ob = bj ? j0 + lo < N && k0 + h < kend : j0 + h < N && k0 + lo < kend;
+            ra[r] = oa ? pa[r * da] : 0.f;
+            rb[r] = ob ? to_f<TB>(pb[r * db]) : 0.f;
         }
+        pa += na;
+        pb += nb;
     };
-    float acc[4][2];
-#pragma unroll
-    for (int a = 0; a < 4; a++) acc[a][0] = acc[a][1] = 0.f;
+    float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
     if (kbeg < kend) fetch(kbeg);
     for (int k0 = kbeg; k0 < kend; k0 += BK) {
         __syncthreads();   // the tiles in shared memory are used up
 #pragma unroll
         for (int r = 0; r < PT; r++) {
-            const int e = tid + GT * r, hi = e / 32, lo = e % 32;
-            As[ak ? lo : hi][ak ? hi : lo] = ra[r];
-            Bs[bj ? hi : lo][bj ? lo : hi] = rb[r];
+            const int h = hi + PS * r;
+            As[ak ? lo : h][ak ? h : lo] = ra[r];
+            Bs[bj ? h : lo][bj ? lo : h] = rb[r];
         }
         __syncthreads();
         if (k0 + BK < kend) fetch(k0 + BK);
 #pragma unroll
         for (int kk = 0; kk < BK; kk++) {
-            const float4 x = *reinterpret_cast<const float4 *>(&As[kk][4 * ty]);
+            const float2 x = *reinterpret_cast<const float2 *>(&As[kk][2 * ty]);
             const float2 y = *reinterpret_cast<const float2 *>(&Bs[kk][2 * tx]);
             acc[0][0] = fmaf(x.x, y.x, acc[0][0]);
             acc[0][1] = fmaf(x.x, y.y, acc[0][1]);
             acc[1][0] = fmaf(x.y, y.x, acc[1][0]);
             acc[1][1] = fmaf(x.y, y.y, acc[1][1]);
-            acc[2][0] = fmaf(x.z, y.x, acc[2][0]);
-            acc[2][1] = fmaf(x.z, y.y, acc[2][1]);
-            acc[3][0] = fmaf(x.w, y.x, acc[3][0]);
-            acc[3][1] = fmaf(x.w, y.y, acc[3][1]);
         }
     }
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int a = 0; a < 2; a++)
 #pragma unroll
         for (int b = 0; b < 2; b++) {
-            const int i = i0 + ty * 4 + a, j = j0 + tx * 2 + b;
+            const int i = i0 + ty * 2 + a, j = j0 + tx * 2 + b;
             if (i >= M || j >= N) continue;
             const long o = (long)i * ldc + j;
             if (EPI == EPI_FWD_HIDDEN) {
