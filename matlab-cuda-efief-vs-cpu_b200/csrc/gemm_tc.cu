@@ -70,11 +70,14 @@ struct Tile {
     static constexpr int UH = BN / 2;                           // U columns per CTA
     static constexpr int USUB = UH * KC;                        // halves per U component sub-tile
     static constexpr int STAGE = CHUNK_HALVES + 4 * USUB;       // L chunk + U half chunk
-    // stages of the ring: 192 KB for BN = 256 (one CTA per SM); 96 KB for
-    // BN = 128, so that two CTAs (pairs) share an SM and one's set-up, drain
-    // and reductions overlap the other's MMAs (2 x 256 TMEM columns)
-    static constexpr int NST = BN == 256 ? 3 : 2;
-    static constexpr int CTAS = BN == 256 ? 1 : 2;              // CTAs per SM
+    // stages of the ring: 192 KB either way, so that an SM holds one CTA.  Two
+    // pairs on one pair of SMs (BN = 128 with two stages) may each get their
+    // TMEM allocation started on the other SM first: a cta_group::2
+    // allocation holds its SM's permit while it waits for its peer, so the
+    // two wait for one another and neither ever returns.  Rare (a sweep in
+    // thousands), but no bounded wait covers it.
+    static constexpr int NST = BN == 256 ? 3 : 4;
+    static constexpr int CTAS = 1;                              // CTAs per SM
     // 4 KB reduction tiles per epilogue warp in the freed stages (at most 4)
     static constexpr int ER = (int)(NST * STAGE * sizeof(__half) / (8 * 4096)) < 4
                                   ? (int)(NST * STAGE * sizeof(__half) / (8 * 4096))

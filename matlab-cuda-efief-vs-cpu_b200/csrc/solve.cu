@@ -1020,6 +1020,8 @@ efie_status efie_mixed_workspace(SolveWork &w, int N, int B, int kb_outer) {
     w.fsrc_on = false;
     EFIE_TRY(efie_trsv_workspace(w));
     EFIE_TRY(efie_gemm_workspace(w));
+    // the zero fills above run on the legacy stream, which the plan's streams do not wait for
+    EFIE_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
     if (!w.hi) {
         int least = 0, greatest = 0;
         EFIE_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
