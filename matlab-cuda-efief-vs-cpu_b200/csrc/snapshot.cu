@@ -32,56 +32,71 @@ constexpr int KMAX = EFIE_SNAP_MAX;   // snapshots per frequency
 static_assert(KMAX == 23, "the wider QR holds 24 columns");
 
 // ---------------------------------------------------------------------------
-// W_f = Z_f X_f for up to K vectors, Z symmetric (upper triangle and full
+// W_f = Z_f X_f for up to 8 NG vectors, Z symmetric (upper triangle and full
 // 128 x 128 diagonal blocks stored).  An item is a block of 128 rows I of one
 // frequency: its y_I stays in registers over all blocks J, from tile (I, J)
 // as stored for J >= I and from the stored tile (J, I) transposed below, so
 // there are no partial vectors and no sums across tiles; Z is read twice
 // (once from L2 where the two readers meet), which the FP64 pipe hides: a
-// 64 KB chunk costs 64 K multiply-adds per lane, as long as HBM takes for it
-// at K = 12.  Chunks are 32 of the contraction's entries, through a ring of
-// three stages: boxes of 8 rows (128 bytes) in the 128-byte swizzle, so that
-// eight lanes on eight rows of one column (as stored) and on eight columns of
-// one row (transposed) both touch eight different 16-byte banks.  Lane
-// (l & 7, l >> 3) of warp w owns y_I[8 w + (l & 7)] over every fourth entry;
-// the X slices of the chunk come with it in the stage.  Ne 6968, 22
-// frequencies, 15 vectors: 7.3 ms, 55 % of the FP64 pipe; eight warps with two
-// rows per lane took 7.9 (two warps per scheduler wait for shared memory), one
-// broadcast entry of X per read with a feeding warp 7.4.
+// 64 KB chunk of 16 vectors costs 2048 multiply-adds per lane of the SM's 128.
+// Chunks are 32 of the contraction's entries, through a ring of three stages:
+// boxes of 8 rows (128 bytes) in the 128-byte swizzle.
+// The products are FP64 matrix instructions (16 x 8 x 8): warp w forms rows
+// 16 (w & 7) .. + 15 of eight vectors, four products per step (re re, re im,
+// -im im, im re) from six shared-memory reads, where a lane that forms its
+// own row reads every vector's entry for four multiply-adds.  Row r of an
+// eight-row box is held by lane group 2 (r & 3) + (r >> 2), so that the eight
+// lanes of a shared-memory phase (two groups x four contraction entries) meet
+// eight different 16-byte banks of the swizzle, as stored and transposed;
+// the vectors' slices are 64 bytes apart modulo 128 for the same reason.
+// One more warp issues the copies.  Bound by the FP64 pipe: Ne 6968, 22
+// frequencies, 15 vectors: 5.05 ms, 76 % of it (nine rounds of items over the
+// SMs where 8.2 would do); one row per lane of sixteen warps with plain
+// multiply-adds took 7.3 ms.
 // ---------------------------------------------------------------------------
 constexpr int MB = 128;                             // rows per item
 constexpr int MC = 32;                              // contraction entries per chunk
 constexpr int MR = 3;                               // stages
-constexpr int MT = 512;                             // threads
 constexpr uint32_t MZ = MB * MC * sizeof(double2);  // 64 KB of Z per chunk
-constexpr uint32_t MX = MC * sizeof(double2);       // one vector's slice
+constexpr uint32_t MX = MC * sizeof(double2) + 64;  // one vector's slice
 
-template <int K>
-constexpr size_t multi_smem() {
-    return MR * (size_t)(MZ + K * MX) + 1024 + 64;
+template <int NG>   // the swizzle follows address bits: stages start on 1024 bytes
+constexpr uint32_t multi_stage = (MZ + 8 * NG * MX + 1023u) & ~1023u;
+template <int NG>
+constexpr size_t multi_smem = MR * (size_t)multi_stage<NG> + 1024 + 64;
+
+// d += a b on 16 x 8 x 8: a row major, b column major
+__device__ __forceinline__ void dmma(double (&d)[4], const double (&a)[4], const double (&b)[2]) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
 struct SnapIdx {
     const int *k;     // [nf] snapshots of each frequency
     const int *pos;   // [nf][KMAX] their rows of xall, nearest first
-};   // a launch takes vectors v0 .. v0 + K - 1 into those columns of W [nf][ldw][N]
+};   // a launch takes vectors v0 .. v0 + 8 NG - 1 into those columns of W [nf][ldw][N]
 
-template <int K>
-__global__ void __launch_bounds__(MT, 1) k_symv_multi(const __grid_constant__ CUtensorMap dmap,
+template <int NG>
+__global__ void __launch_bounds__(256 * NG + 32, 1) k_symv_multi(const __grid_constant__ CUtensorMap dmap,
                                                        const __grid_constant__ CUtensorMap tmap, int N, int nb, int nf,
                                                        const double2 *__restrict__ xall, const SnapIdx S,
                                                        double2 *__restrict__ W, int v0, int ldw, char *ctl) {
     extern __shared__ unsigned char dsm[];
     __shared__ int fail;
-    constexpr uint32_t STAGE = MZ + K * MX;
+    constexpr int K = 8 * NG, MT = 256 * NG + 32;
+    constexpr uint32_t STAGE = multi_stage<NG>;
     unsigned char *ring = dsm + (((smem_u32(dsm) + 1023u) & ~1023u) - smem_u32(dsm));
     uint64_t *full = reinterpret_cast<uint64_t *>(ring + MR * STAGE);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool feeder = warp == 8 * NG;   // the last warp issues the copies
     const int G = gridDim.x, items = nb * nf;
     // slices past row N are not copied: what a stage holds there must be finite
-    for (int i = tid; i < MR * K * MC; i += MT)
-        reinterpret_cast<double2 *>(ring + (i / (K * MC)) * STAGE + MZ)[i % (K * MC)] = make_double2(0.0, 0.0);
-    int p_it = blockIdx.x, p_q = 0, issued = 0;   // producer (thread 0): chunk p_q of item p_it is next
+    constexpr int NX = K * (int)(MX / sizeof(double2));
+    for (int i = tid; i < MR * NX; i += MT)
+        reinterpret_cast<double2 *>(ring + (i / NX) * STAGE + MZ)[i % NX] = make_double2(0.0, 0.0);
+    int p_it = blockIdx.x, p_q = 0, issued = 0;   // producer (feeder's lane 0): chunk p_q of item p_it is next
     auto produce = [&]() {
         if (p_it >= items) return;
         const int f = p_it / nb, I = p_it - f * nb, J = p_q >> 2, n0 = J * MB + (p_q & 3) * MC;
@@ -107,60 +122,59 @@ __global__ void __launch_bounds__(MT, 1) k_symv_multi(const __grid_constant__ CU
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the zeros before the copies
     __syncthreads();
-    if (tid == 0)
+    if (feeder && lane == 0)
         for (int s = 0; s < MR; s++) produce();
-    const int li = lane & 7, g = lane >> 3;
+    const int g = lane >> 2, t = lane & 3, row = (g & 1) * 4 + (g >> 1), w8 = warp & 7, v8 = 8 * (warp >> 3);
     int cc = 0;
     for (int it = blockIdx.x; it < items; it += G) {
         const int f = it / nb, I = it - f * nb;
-        double2 acc[K];
-#pragma unroll
-        for (int v = 0; v < K; v++) acc[v] = make_double2(0.0, 0.0);
+        double yr[4] = {0.0, 0.0, 0.0, 0.0}, yi[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 1
         for (int q = 0; q < 4 * nb; q++) {
-            if (!mbar_wait_bounded(full + cc % MR, (uint32_t)(cc / MR) & 1u)) fail = 1;
+            if (!feeder && !mbar_wait_bounded(full + cc % MR, (uint32_t)(cc / MR) & 1u)) fail = 1;
             const unsigned char *st = ring + (cc % MR) * STAGE;
-            if (!fail) {
-                const double2 *X = reinterpret_cast<const double2 *>(st + MZ) + g;
-                // the entry of contraction index 4 c8 + g: box, row and 16-byte
-                // chunk of the swizzle as stored, or transposed (block-uniform)
+            if (!feeder && __all_sync(0xffffffffu, !fail)) {   // matrix instructions want whole warps
+                const unsigned char *X = st + MZ + (v8 + g) * MX + t * sizeof(double2);
+                // rows r and r + 8 of the warp, contraction entries c = 8 k + t and + 4: box,
+                // row and 16-byte chunk of the swizzle as stored, or transposed (block-uniform)
                 const bool direct = (q >> 2) >= I;
-                const unsigned char *zb = direct ? st + warp * 4096 + g * 128 : st + (8 * warp + li) * 128;
-#pragma unroll 2
-                for (int c8 = 0; c8 < MC / 4; c8++) {
-                    const int h = (c8 & 1) * 4 + g;   // contraction index mod 8
-                    const unsigned char *p = zb + (direct ? c8 * 512 : (c8 >> 1) * 16384) + ((li ^ h) << 4);
-                    const double2 a = *reinterpret_cast<const double2 *>(p);
+                const unsigned char *zb = direct ? st + w8 * 8192 + t * 128 : st + (16 * w8 + row) * 128;
+                const int r8 = direct ? 4096 : 1024, c4 = direct ? 512 : 0, c8 = direct ? 1024 : 16384;
+                const int x0 = (row ^ t) << 4, x4 = x0 ^ 64;
 #pragma unroll
-                    for (int v = 0; v < K; v++) {
-                        const double2 x = X[v * MC + 4 * c8];
-                        acc[v].x = fma(a.x, x.x, fma(-a.y, x.y, acc[v].x));
-                        acc[v].y = fma(a.x, x.y, fma(a.y, x.x, acc[v].y));
-                    }
+                for (int k = 0; k < MC / 8; k++) {
+                    const unsigned char *p = zb + k * c8;
+                    const double2 a0 = *reinterpret_cast<const double2 *>(p + x0);
+                    const double2 a1 = *reinterpret_cast<const double2 *>(p + r8 + x0);
+                    const double2 a2 = *reinterpret_cast<const double2 *>(p + c4 + x4);
+                    const double2 a3 = *reinterpret_cast<const double2 *>(p + r8 + c4 + x4);
+                    const double2 b0 = *reinterpret_cast<const double2 *>(X + k * 128);
+                    const double2 b1 = *reinterpret_cast<const double2 *>(X + k * 128 + 64);
+                    const double zr[4] = {a0.x, a1.x, a2.x, a3.x}, zi[4] = {a0.y, a1.y, a2.y, a3.y};
+                    const double xr[2] = {b0.x, b1.x}, xi[2] = {b0.y, b1.y}, xn[2] = {-b0.y, -b1.y};
+                    dmma(yr, zr, xr);
+                    dmma(yi, zr, xi);
+                    dmma(yr, zi, xn);
+                    dmma(yi, zi, xr);
                 }
             }
             __syncthreads();   // every warp is done with the stage
             if (fail) {
                 // a chunk never arrived: every frequency of the launch falls back
                 if (tid < nf) atomicExch(reinterpret_cast<int *>(ctl + 64 * tid + 36), 3);
-                if (tid == 0)
+                if (feeder && lane == 0)
                     for (int k = cc + 1; k < issued; k++)
                         if (!mbar_wait_bounded(full + k % MR, (uint32_t)(k / MR) & 1u)) break;
                 return;
             }
-            if (tid == 0) produce();
+            if (feeder && lane == 0) produce();
             cc++;
         }
-        const int m = I * MB + 8 * warp + li;
+        if (feeder) continue;
 #pragma unroll
-        for (int v = 0; v < K; v++) {
-            double2 s = acc[v];
-#pragma unroll
-            for (int o = 8; o <= 16; o <<= 1) {
-                s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-                s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
-            }
-            if (g == (v & 3) && m < N && v0 + v < ldw) W[((size_t)f * ldw + v0 + v) * N + m] = s;
+        for (int i = 0; i < 4; i++) {
+            const int m = I * MB + 16 * w8 + 8 * (i >> 1) + row, v = v0 + v8 + 2 * t + (i & 1);
+            if (m < N && v < ldw) W[((size_t)f * ldw + v) * N + m] = make_double2(yr[i], yi[i]);
         }
     }
 }
@@ -333,12 +347,12 @@ efie_status multi_maps(int N, int B, const void *Z, size_t zstride, CUtensorMap 
                              CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-template <int K>
+template <int NG>
 efie_status launch_multi(efie_ctx *ctx, const CUtensorMap &d, const CUtensorMap &t, int N, int nf,
                          const double2 *xall, const SnapIdx &S, double2 *W, int v0, int ldw, char *ctl) {
     const int nb = (N + MB - 1) / MB;
-    EFIE_CUDA(cudaFuncSetAttribute(k_symv_multi<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)multi_smem<K>()));
-    k_symv_multi<K><<<std::min(ctx->num_sms, nb * nf), MT, multi_smem<K>(), ctx->stream>>>(d, t, N, nb, nf, xall, S, W,
+    EFIE_CUDA(cudaFuncSetAttribute(k_symv_multi<NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)multi_smem<NG>));
+    k_symv_multi<NG><<<std::min(ctx->num_sms, nb * nf), 256 * NG + 32, multi_smem<NG>, ctx->stream>>>(d, t, N, nb, nf, xall, S, W,
                                                                                            v0, ldw, ctl);
     return efie_cuda_check(cudaGetLastError(), "snapshot products");
 }
@@ -352,8 +366,8 @@ efie_status efie_snapshot_guess(efie_ctx *ctx, SolveWork &w, const void *Z, size
     int kmax = 0;
     for (int f = 0; f < nf; f++) kmax = std::max(kmax, spec.k[f]);
     if (nf < 1 || kmax < 1 || kmax > KMAX) return efie_fail(EFIE_ERR_ARGS, "snapshot guess: bad snapshot count");
-    // vectors per product launch; up to 15 snapshots go in one, more in two of twelve
-    const int ldw = kmax <= 4 ? 4 : kmax <= 8 ? 8 : kmax <= 12 ? 12 : kmax <= 15 ? 15 : 23;
+    // up to eight or sixteen vectors per product launch
+    const int ldw = kmax <= 8 ? 8 : kmax <= 15 ? 15 : 23;
     const int QC = ldw <= 15 ? 16 : 24;
     // W [nf][ldw][N], R [nf][nblk][QC][QC], coefficients [nf][KMAX], spec
     const size_t nW = (size_t)nf * ldw * N, nR = (size_t)nf * nblk * QC * QC, nC = (size_t)nf * KMAX;
@@ -367,15 +381,10 @@ efie_status efie_snapshot_guess(efie_ctx *ctx, SolveWork &w, const void *Z, size
     EFIE_TRY(multi_maps(N, w.B, Z, zstride, &d, &t));
     size_t tok = ctx->log.begin(s);
     char *ctl = w.ctl.as<char>();
-    switch (ldw) {
-    case 4: EFIE_TRY(launch_multi<4>(ctx, d, t, N, nf, xa, S, W, 0, ldw, ctl)); break;
-    case 8: EFIE_TRY(launch_multi<8>(ctx, d, t, N, nf, xa, S, W, 0, ldw, ctl)); break;
-    case 12: EFIE_TRY(launch_multi<12>(ctx, d, t, N, nf, xa, S, W, 0, ldw, ctl)); break;
-    case 15: EFIE_TRY(launch_multi<16>(ctx, d, t, N, nf, xa, S, W, 0, ldw, ctl)); break;
-    default:
-        EFIE_TRY(launch_multi<12>(ctx, d, t, N, nf, xa, S, W, 0, ldw, ctl));
-        EFIE_TRY(launch_multi<12>(ctx, d, t, N, nf, xa, S, W, 12, ldw, ctl));
-    }
+    if (ldw > 8)
+        EFIE_TRY(launch_multi<2>(ctx, d, t, N, nf, xa, S, W, 0, ldw, ctl));
+    if (ldw != 15)
+        EFIE_TRY(launch_multi<1>(ctx, d, t, N, nf, xa, S, W, ldw > 8 ? 16 : 0, ldw, ctl));
     const int nprod = ldw > 15 ? 2 : 1;
     ctx->log.end(EFIE_K_RESIDUAL, s, tok, nprod * 8.0 * (double)N * N * nf, nprod);
     tok = ctx->log.begin(s);
