@@ -22,10 +22,10 @@
 // moments once and writes every frequency's entry: an entry and frequency
 // cost about 2 N + 30 FP64 instructions and its 16 bytes of Z instead of nine
 // point pairs' phases, a pair value written to memory and four read back.
-// Measured (one B200, 3-point rule, Ne 6968, N = 10): 5.0 ms per sweep and
-// 0.15 ms per frequency, against 1.22 ms per frequency with the pair values;
+// Measured (one B200, 3-point rule, Ne 6968, N = 12): 4.7 ms per sweep and
+// 0.18 ms per frequency, against 1.22 ms per frequency with the pair values;
 // 6-point rule with 9216-point-pair near pairs, Ne 1074, 21 frequencies:
-// 5.8 ms against 54.
+// 2.6 ms against 54.
 #include <algorithm>
 #include <cmath>
 #include <complex>
@@ -308,7 +308,9 @@ __global__ void __launch_bounds__(64) k_series_adjacent(const SpecialArgs q, dou
 // conflict-free ([component][row] in shared memory).  A thread holds the 2 N
 // sums in registers over the entry's up to four triangle pairs; the powers of
 // t run in two chains (even and odd) to halve the dependent multiplications.
-// Bound by the FP64 pipe: about 24 + 3 N instructions per point pair.
+// Bound by the FP64 pipe: about 24 + 3 N instructions per point pair, at N = 12
+// 83 operations by the counters and 18.2 TFLOP/s (Ne 4110: 1.42 ms), half of
+// what cuBLAS DGEMM reaches with nothing but fused multiply-adds.
 // mom[((tile - tile0) * 2 N + comp) * 1024 + column * 32 + row], comp = A_0.., S_0...
 // ---------------------------------------------------------------------------
 template <int NQ>
