@@ -973,7 +973,8 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
     const int wanted = snapshots_wanted(Nf > 0 ? (kmax - kmin) * p->extent : 0.0);
     // a sweep of no more frequencies than may be factored is one batch
     const int na = Nf <= choose_anchors(N) ? Nf : std::min(wanted, choose_anchors(N));
-    const bool anchored = refines && p->auto_share && p->sw.zsym && p->sw.sym_lu && na <= B;
+    // (an empty list has no batch)
+    const bool anchored = Nf > 0 && refines && p->auto_share && p->sw.zsym && p->sw.sym_lu && na <= B;
     const int lvl1 = anchored && na < wanted && Nf - na > 2 * (wanted - na) ? std::min(B, wanted - na) : 0;
     const int tail = anchored ? (Nf - na - lvl1 + B - 1) / B : 0;   // batches of the remaining frequencies
     const int nbat = anchored ? 1 + (lvl1 > 0) + tail : (Nf + B - 1) / B;
