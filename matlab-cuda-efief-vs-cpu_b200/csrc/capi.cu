@@ -927,6 +927,18 @@ static bool snapshot_nodes(const int *pos, int nb, const std::vector<double> &fs
     return true;
 }
 
+// What a sweep on shared factors solves to, as a part of the residual target
+// (efie_mixed_gmres: aim).  The frequencies of its first batch become the snapshots
+// every later start is a combination of, so their errors enter all of them;
+// the others end on a neighbour's factors, or on no step at all, and such a
+// residual of half the target leaves more error in the currents than one
+// that the frequency's own factors have brought there.  Measured against the
+// complex128 solver (37 sweeps, Ne 500 to 20000; the worst and the median
+// current errors, geometric means over them): 1.45 and 1.58 times those of
+// interpolated starts at half the target for all, 0.51 and 0.78 times with
+// these; it costs 3 % of the time (Ne 6968, 101 frequencies: 86.5 -> 95 ms).
+constexpr double kAimSnapshots = 0.02, kAimShared = 0.1, kAim = 0.5;
+
 static bool g_warm_start_disabled = false;
 extern "C" void efie_debug_disable_warm_start(int disable) { g_warm_start_disabled = disable != 0; }
 
@@ -1153,7 +1165,8 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
                                        p->opts.refine_max_iter, active, &rr);
             else
                 rc = efie_mixed_gmres(ctx, p->sw, p->Z.p, NN, p->b.p, p->x.p, p->bnorm, p->opts.refine_tol,
-                                      p->opts.refine_max_iter, active, &rr, guess);
+                                      p->opts.refine_max_iter, active, &rr, guess,
+                                      !share ? kAim : bi == 0 ? kAimSnapshots : kAimShared);
             if (rc != EFIE_OK) break;
             S->refine_iters_max = std::max(S->refine_iters_max, rr.iters);
             int err1[EFIE_MAX_BATCH];   // device error codes of the first attempt

@@ -589,7 +589,7 @@ efie_status gm_workspace(SolveWork &w) {
 
 efie_status efie_mixed_gmres(efie_ctx *ctx, SolveWork &w, const void *Z, size_t zstride, const void *b, void *x,
                              double bnorm, double tol, int max_iter, const int *active_host, RefineResult *res,
-                             bool x0_given) {
+                             bool x0_given, double aim) {
     cudaStream_t s = ctx->stream;
     KernelLog &log = ctx->log;
     const int N = w.N, B = w.B;
@@ -605,7 +605,7 @@ efie_status efie_mixed_gmres(efie_ctx *ctx, SolveWork &w, const void *Z, size_t 
     int nact = 0;
     for (int f = 0; f < B; f++) nact += active_host[f] ? 1 : 0;
     const double zbytes = 16.0 * (double)N * N, lubytes = 8.0 * (double)N * N;
-    const double tol_inner = 0.5 * tol;
+    const double tol_inner = aim * tol;
     const int *ctl_skip0 = reinterpret_cast<const int *>(ctl + 32);   // ctl skip flag of slot f: [16 f]
     auto residual = [&](double done) -> efie_status {   // done: the norm that counts as solved
         if (!w.zsym) return efie_true_residual(ctx, w, Z, zstride, x, b, done, V, nact);

@@ -129,9 +129,11 @@ efie_status efie_mixed_refine(efie_ctx *ctx, SolveWork &w, const void *Z, size_t
 // the Arnoldi process and every vector are complex128.  Same contract as
 // efie_mixed_refine (x starts at 0; res->iters counts matrix-vector products).
 // x0_given: the active slots of x hold initial guesses (x = 0 otherwise).
+// aim: the cycles stop, and a guess passes without one, at aim * tol; what
+// counts as solved is the true residual at tol.
 efie_status efie_mixed_gmres(efie_ctx *ctx, SolveWork &w, const void *Z, size_t zstride, const void *b, void *x,
                              double bnorm, double tol, int max_iter, const int *active_host, RefineResult *res,
-                             bool x0_given = false);
+                             bool x0_given = false, double aim = 0.5);
 // r = b - Z x for every frequency of the batch (complex128), its complex64
 // copy in w.vec, ||r|| / ||b|| and the convergence flags in w.ctl; r is also
 // stored at rout + N f when rout is not null.
