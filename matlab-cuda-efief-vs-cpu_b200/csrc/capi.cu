@@ -1079,12 +1079,14 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
     // the plan's slots; each is refined with the factors of the nearest of
     // them (its assembly then leaves the planes alone).  GMRES converges to
     // the same residual target in a few more steps; a frequency that does
-    // not gets the retry below, with its own factors -- which converts Z to
-    // planes in every slot, so the rest of the group then factors itself.
+    // not gets the retry below, whose factors take its own slot's place among
+    // those that later batches choose from.
     const int group = anchored ? nbat : p->share_group;   // batches per factored batch
     const bool share = mixed && warm && group > 1 && p->sw.zsym && p->sw.sym_lu &&
                        p->opts.refine_method == EFIE_REFINE_GMRES;
-    bool prev_factored = false;      // the slots hold the factors of the group's first batch
+    constexpr double kNone = -1.0;                  // frequencies are positive
+    std::vector<double> held(p->B, kNone);          // the frequency whose factors each slot holds
+    auto any_held = [&] { return std::any_of(held.begin(), held.end(), [](double h) { return h > 0.0; }); };
     std::vector<int> fsrc_host(p->B);
     p->sw.fsrc_on = false;
     auto set_fsrc = [&](bool identity) -> efie_status {
@@ -1103,7 +1105,7 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
         const int f0 = bstart[bi], nb = bstart[bi + 1] - f0;
         int active[EFIE_MAX_BATCH] = {0};
         for (int f = 0; f < nb; f++) active[f] = 1;
-        const bool shared = share && (bi % group) != 0 && prev_factored;
+        const bool shared = share && (bi % group) != 0 && any_held();
         {
             Physics ph[EFIE_MAX_BATCH];
             void *Zf[EFIE_MAX_BATCH];
@@ -1125,15 +1127,14 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
         bool fallback[EFIE_MAX_BATCH] = {false};
         if (mixed) {
             if (shared) {
-                // each slot refines with the factors of the group's factored
-                // batch's slot holding the nearest frequency
-                const int gb = bi - bi % group, p0 = bstart[gb], np_ = bstart[gb + 1] - p0;
+                // each slot refines with the factors of the slot that holds
+                // the nearest frequency's
                 for (int f = 0; f < p->B; f++) fsrc_host[f] = f;
                 for (int f = 0; f < nb; f++) {
-                    int best = 0;
+                    int best = -1;
                     const double fq = fsorted[posq[f0 + f]];
-                    for (int s2 = 1; s2 < np_; s2++)
-                        if (std::abs(fsorted[posq[p0 + s2]] - fq) < std::abs(fsorted[posq[p0 + best]] - fq)) best = s2;
+                    for (int s2 = 0; s2 < p->B; s2++)
+                        if (held[s2] > 0.0 && (best < 0 || std::abs(held[s2] - fq) < std::abs(held[best] - fq))) best = s2;
                     fsrc_host[f] = best;
                 }
                 rc = set_fsrc(false);
@@ -1142,9 +1143,9 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
             } else {
                 rc = set_fsrc(true);
                 if (rc == EFIE_OK) rc = plan_factor(p, active, nb);
+                for (int f = 0; f < p->B; f++) held[f] = f < nb ? fsorted[posq[f0 + f]] : kNone;
             }
             if (rc != EFIE_OK) break;
-            if (!shared && bi % group == 0) prev_factored = true;
             RefineResult rr;
             const bool guess = warm && bi > 0;
             SnapSpec sp;
@@ -1182,11 +1183,10 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
                 if (nr > 0) {
                     RefineResult r2;
                     const bool pfa = p->sw.planes_from_assembly;
-                    // the retried frequencies refine with their own factors;
-                    // the slots no longer hold the group's factors
+                    // the retried frequencies refine with their own factors
                     rc = set_fsrc(true);
                     if (rc != EFIE_OK) break;
-                    prev_factored = false;
+                    if (shared) S->n_shared_factors -= nr;
                     // the general LU converts all of Z
                     for (int f = 0; f < nb && rc == EFIE_OK; f++)
                         if (retry[f] && pfa) rc = efie_z_mirror(ctx, Zslot(f), N);
@@ -1202,7 +1202,10 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
                     if (rc != EFIE_OK) break;
                     S->refine_iters_max = std::max(S->refine_iters_max, r2.iters);
                     for (int f = 0; f < nb; f++)
-                        if (retry[f]) rr.relres[f] = r2.relres[f], rr.converged[f] = r2.converged[f], rr.err[f] = r2.err[f];
+                        if (retry[f]) {
+                            rr.relres[f] = r2.relres[f], rr.converged[f] = r2.converged[f], rr.err[f] = r2.err[f];
+                            held[f] = rr.converged[f] && !rr.err[f] ? fsorted[posq[f0 + f]] : kNone;
+                        }
                 }
             }
             for (int f = 0; f < nb; f++) {

@@ -43,9 +43,11 @@ __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
 // Z_f (c128, column-major) -> planes_f (row-major).  32x32 tiles, grid z = f.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_z_to_planes(int N, const double2 *__restrict__ Z, size_t zstride,
-                                                     float *__restrict__ planes, size_t pstride, int ld) {
+                                                     float *__restrict__ planes, size_t pstride, int ld,
+                                                     const int *__restrict__ active) {
     __shared__ float tr[32][33], ti[32][33];
     const int f = blockIdx.z;
+    if (!active[f]) return;   // the slot keeps its factors
     Z += zstride * f;
     float *Ar = planes + pstride * f, *Ai = Ar + (size_t)ld * N;
     const int bx = blockIdx.x * 32, by = blockIdx.y * 32;  // bx: column block, by: row block
@@ -1089,7 +1091,7 @@ efie_status efie_mixed_factor_launch(efie_ctx *ctx, SolveWork &w, const void *Z,
             for (int f = 0; f < B; f++)
                 EFIE_TRY(efie_z_mirror(ctx, static_cast<double2 *>(const_cast<void *>(Z)) + zstride * f, N));
         tok = log.begin(s0);
-        k_z_to_planes<<<tg, 256, 0, s0>>>(N, static_cast<const double2 *>(Z), zstride, planes, w.pstride, ld);
+        k_z_to_planes<<<tg, 256, 0, s0>>>(N, static_cast<const double2 *>(Z), zstride, planes, w.pstride, ld, active);
         EFIE_CUDA(cudaGetLastError());
         log.end(EFIE_K_PANEL, s0, tok, 24.0 * (double)N * N * nact);
     }
