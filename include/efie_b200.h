@@ -16,6 +16,7 @@
 #ifndef EFIE_B200_H
 #define EFIE_B200_H
 
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
@@ -411,6 +412,11 @@ void efie_debug_set_selftest_tiles(int tile_chain, int tile_bulk, int resident);
  * guesses interpolated from the solved neighbours (mixed solver, GMRES, more
  * than one batch), process-wide.  No counterpart in the reference. */
 void efie_debug_disable_warm_start(int disable);
+
+/* Test hook: device allocations of more than max_bytes fail as they do when
+ * the memory is taken (0: none do), process-wide.  No counterpart in the
+ * reference. */
+void efie_debug_limit_allocations(size_t max_bytes);
 
 /* Z of nf (at most the plan's batch) frequencies as a sweep assembles them
  * from frequency-independent moments, Z[nf][Ne x Ne] column-major on the

@@ -1149,8 +1149,9 @@ namespace {
 // edge combinations or the 8 moments) for up to four frequencies assembled
 // together, within a quarter of free memory or the buffer at hand.
 efie_status pair_values(GeomDev &g) {
-    if (g.mf > 0) return EFIE_OK;
     const size_t per = sizeof(double2) * (g.combo ? 9 : 8) * g.npairs;
+    if (g.mf > 0 && g.moments.bytes >= per * g.mf) return EFIE_OK;   // a series sweep may have changed the buffer
+    g.mf = 0;
     size_t freeb = 0, totalb = 0;
     int mf = 1;
     if ((g.Nq == 3 || g.Nq == 7) && cudaMemGetInfo(&freeb, &totalb) == cudaSuccess)

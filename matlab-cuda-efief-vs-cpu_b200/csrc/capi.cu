@@ -157,7 +157,15 @@ void trim_locked(DevicePool &P) {
 
 }  // namespace
 
+static std::atomic<size_t> g_alloc_limit{0};   // 0: none (efie_debug_limit_allocations)
+extern "C" void efie_debug_limit_allocations(size_t max_bytes) { g_alloc_limit = max_bytes; }
+
 void *efie_pool_get(size_t n, size_t *got, cudaError_t *err) {
+    const size_t limit = g_alloc_limit;
+    if (limit && n > limit) {
+        if (err) *err = cudaErrorMemoryAllocation;
+        return nullptr;
+    }
     int dev = 0;
     cudaGetDevice(&dev);
     {

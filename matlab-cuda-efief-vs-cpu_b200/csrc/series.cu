@@ -850,10 +850,9 @@ efie_status efie_series_begin(efie_ctx *ctx, GeomDev &g, double kabs, double kim
         if (want > old) {
             EFIE_CUDA(cudaStreamSynchronize(s));   // an earlier assembly may still read it
             g.moments.release();
-            if (g.moments.reserve(want) != EFIE_OK) {
-                if (old) EFIE_TRY(g.moments.reserve(old));
-                return EFIE_OK;
-            }
+            g.mf = 0;
+            // no room after all: the sweep takes the pair values, which reserve what they need
+            if (g.moments.reserve(want) != EFIE_OK) return EFIE_OK;
         }
     }
     const size_t cap = g.moments.bytes / per;
