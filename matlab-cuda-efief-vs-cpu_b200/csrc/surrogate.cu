@@ -29,8 +29,7 @@
 
 namespace {
 
-constexpr int BM = 32, BN = 32, BK = 32;
-constexpr int GT = 256;   // threads of a product's CTA, 2 x 2 outputs each
+constexpr int GT = 256;   // threads of a product's CTA
 
 enum Epilogue { EPI_FWD_HIDDEN = 0, EPI_FWD_OUT = 1, EPI_BWD_DZ = 2, EPI_PARTIAL = 3 };
 constexpr int KSPLIT = 512;   // K chunk of the weight-gradient products
@@ -50,69 +49,83 @@ __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return _
 // kchunk; EPI_PARTIAL stores chunk z's partial product at C + z M ldc, and
 // k_sum_parts adds the chunks in order (bit-reproducible gradients).
 //
-// The layers are small (1024 x 256 x 256), so a product is bound by latency:
-// 32 x 32 tiles fill the GPU (256 CTAs for a layer; 64 x 64 tiles left half of
-// the SMs idle), and the next 32 of K are read into registers while the
-// current ones are used.  A training step of five layers of batch 1024 took
-// 480 us with 64 x 64 tiles read between two barriers per 16 of K.
-template <typename TB, int EPI>
-__global__ void __launch_bounds__(GT) k_mlp_gemm(int M, int N, int K, const float *__restrict__ A, long sai,
+// T x T tiles, T / 16 squared outputs per thread; the next tiles are read into
+// registers while the current ones are used.  The layers are small (1024 x
+// 256 x 256), so a product is bound by latency: 32 x 32 tiles fill the GPU
+// (256 CTAs for a layer; 64 x 64 tiles leave half of the SMs idle).  Where 64 x
+// 64 tiles fill it too, each of their operands read from shared memory serves
+// four multiply-adds instead of two.  The sums' order is the same.
+template <typename TB, int EPI, int T>
+__global__ void __launch_bounds__(GT, 4) k_mlp_gemm(int M, int N, int K, const float *__restrict__ A, long sai,
                                                  long sak, const TB *__restrict__ B, long sbk, long sbj,
                                                  float *__restrict__ C, int ldc, const float *__restrict__ bias,
                                                  float *__restrict__ Aout, const float *__restrict__ Zprev,
                                                  int kchunk) {
-    __shared__ __align__(8) float As[BK][BM + 2];
-    __shared__ __align__(8) float Bs[BK][BN + 2];
+    constexpr int R = T / 16, BK = T == 32 ? 32 : 16, PAD = R;   // PAD keeps the rows aligned for R floats
+    __shared__ __align__(16) float As[BK][T + PAD];
+    __shared__ __align__(16) float Bs[BK][T + PAD];
     const int tid = threadIdx.x;
-    const int tx = tid & 15, ty = tid >> 4;   // rows 2 ty, 2 ty + 1, columns 2 tx, 2 tx + 1
-    const int i0 = blockIdx.y * BM, j0 = blockIdx.x * BN;
+    const int tx = tid & 15, ty = tid >> 4;   // rows R ty + a, columns R tx + b
+    const int i0 = blockIdx.y * T, j0 = blockIdx.x * T;
     const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
-    constexpr int PT = BM * BK / GT, PS = GT / 32;   // elements of each tile per thread, their stride
-    const bool ak = sak == 1, bj = sbj == 1;         // contiguous along k, along j
-    const int hi = tid >> 5, lo = tid & 31;
-    const float *pa = A + (long)(i0 + (ak ? hi : lo)) * sai + (long)(kbeg + (ak ? lo : hi)) * sak;
-    const TB *pb = B + (long)(kbeg + (bj ? hi : lo)) * sbk + (long)(j0 + (bj ? lo : hi)) * sbj;
-    const long da = PS * (ak ? sai : sak), db = PS * (bj ? sbk : sbj), na = BK * sak, nb = BK * sbk;
+    constexpr int PT = T * BK / GT;            // elements of each tile per thread
+    const bool ak = sak == 1, bj = sbj == 1;   // contiguous along k, along j
+    // a thread's elements: lo along the contiguous direction, hi + d r along the other
+    const int alo = ak ? tid % BK : tid % T, ahi = ak ? tid / BK : tid / T, ad = ak ? GT / BK : GT / T;
+    const int blo = bj ? tid % T : tid % BK, bhi = bj ? tid / T : tid / BK, bd = bj ? GT / T : GT / BK;
+    const float *pa = A + (long)(i0 + (ak ? ahi : alo)) * sai + (long)(kbeg + (ak ? alo : ahi)) * sak;
+    const TB *pb = B + (long)(kbeg + (bj ? bhi : blo)) * sbk + (long)(j0 + (bj ? blo : bhi)) * sbj;
+    const long da = ad * (ak ? sai : sak), db = bd * (bj ? sbk : sbj), na = BK * sak, nb = BK * sbk;
     float ra[PT], rb[PT];
     auto fetch = [&](int k0) {
 #pragma unroll
         for (int r = 0; r < PT; r++) {
-            const int h = hi + PS * r;
-            const bool oa = ak ? i0 + h < M && k0 + lo < kend : i0 + lo < M && k0 + h < kend;
-            const bool ob = bj ? j0 + lo < N && k0 + h < kend : j0 + h < N && k0 + lo < kend;
+            const int ha = ahi + ad * r, hb = bhi + bd * r;
+            const bool oa = ak ? i0 + ha < M && k0 + alo < kend : i0 + alo < M && k0 + ha < kend;
+            const bool ob = bj ? j0 + blo < N && k0 + hb < kend : j0 + hb < N && k0 + blo < kend;
             ra[r] = oa ? pa[r * da] : 0.f;
             rb[r] = ob ? to_f<TB>(pb[r * db]) : 0.f;
         }
         pa += na;
         pb += nb;
     };
-    float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+    float acc[R][R];
+#pragma unroll
+    for (int a = 0; a < R; a++)
+#pragma unroll
+        for (int b = 0; b < R; b++) acc[a][b] = 0.f;
     if (kbeg < kend) fetch(kbeg);
     for (int k0 = kbeg; k0 < kend; k0 += BK) {
         __syncthreads();   // the tiles in shared memory are used up
 #pragma unroll
         for (int r = 0; r < PT; r++) {
-            const int h = hi + PS * r;
-            As[ak ? lo : h][ak ? h : lo] = ra[r];
-            Bs[bj ? h : lo][bj ? lo : h] = rb[r];
+            const int ha = ahi + ad * r, hb = bhi + bd * r;
+            As[ak ? alo : ha][ak ? ha : alo] = ra[r];
+            Bs[bj ? hb : blo][bj ? blo : hb] = rb[r];
         }
         __syncthreads();
         if (k0 + BK < kend) fetch(k0 + BK);
 #pragma unroll
         for (int kk = 0; kk < BK; kk++) {
-            const float2 x = *reinterpret_cast<const float2 *>(&As[kk][2 * ty]);
-            const float2 y = *reinterpret_cast<const float2 *>(&Bs[kk][2 * tx]);
-            acc[0][0] = fmaf(x.x, y.x, acc[0][0]);
-            acc[0][1] = fmaf(x.x, y.y, acc[0][1]);
-            acc[1][0] = fmaf(x.y, y.x, acc[1][0]);
-            acc[1][1] = fmaf(x.y, y.y, acc[1][1]);
+            float x[R], y[R];
+            if (R == 2) {
+                *reinterpret_cast<float2 *>(x) = *reinterpret_cast<const float2 *>(&As[kk][R * ty]);
+                *reinterpret_cast<float2 *>(y) = *reinterpret_cast<const float2 *>(&Bs[kk][R * tx]);
+            } else {
+                *reinterpret_cast<float4 *>(x) = *reinterpret_cast<const float4 *>(&As[kk][R * ty]);
+                *reinterpret_cast<float4 *>(y) = *reinterpret_cast<const float4 *>(&Bs[kk][R * tx]);
+            }
+#pragma unroll
+            for (int a = 0; a < R; a++)
+#pragma unroll
+                for (int b = 0; b < R; b++) acc[a][b] = fmaf(x[a], y[b], acc[a][b]);
         }
     }
 #pragma unroll
-    for (int a = 0; a < 2; a++)
+    for (int a = 0; a < R; a++)
 #pragma unroll
-        for (int b = 0; b < 2; b++) {
-            const int i = i0 + ty * 2 + a, j = j0 + tx * 2 + b;
+        for (int b = 0; b < R; b++) {
+            const int i = i0 + ty * R + a, j = j0 + tx * R + b;
             if (i >= M || j >= N) continue;
             const long o = (long)i * ldc + j;
             if (EPI == EPI_FWD_HIDDEN) {
@@ -128,6 +141,25 @@ __global__ void __launch_bounds__(GT) k_mlp_gemm(int M, int N, int K, const floa
                 C[(long)blockIdx.z * M * ldc + o] = acc[a][b];
             }
         }
+}
+
+inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
+
+// 64 x 64 tiles where there is one for every SM: a training step of batch 4096
+// (five layers of 256, 256 tiles a product) takes 0.385 ms with them against
+// 0.43 with 32 x 32, one of batch 1024 (64 tiles) 0.28 against 0.17; a
+// prediction of 20480 rows through six layers of 512 takes 2.25 ms against 3.27.
+constexpr long kLargeCtas = 148;
+template <typename TB, int EPI>
+void mlp_gemm(cudaStream_t s, int M, int N, int K, const float *A, long sai, long sak, const TB *B, long sbk, long sbj,
+              float *C, int ldc, const float *bias, float *Aout, const float *Zprev, int kchunk) {
+    const int nz = EPI == EPI_PARTIAL ? cdiv(K, kchunk) : 1;
+    if ((long)cdiv(M, 64) * cdiv(N, 64) * nz >= kLargeCtas)
+        k_mlp_gemm<TB, EPI, 64><<<dim3(cdiv(N, 64), cdiv(M, 64), nz), GT, 0, s>>>(M, N, K, A, sai, sak, B, sbk, sbj, C,
+                                                                                  ldc, bias, Aout, Zprev, kchunk);
+    else
+        k_mlp_gemm<TB, EPI, 32><<<dim3(cdiv(N, 32), cdiv(M, 32), nz), GT, 0, s>>>(M, N, K, A, sai, sak, B, sbk, sbj, C,
+                                                                                  ldc, bias, Aout, Zprev, kchunk);
 }
 
 // out[e] += sum_z part[z * count + e], z in order
@@ -229,7 +261,6 @@ __global__ void k_to_bf16(int n, const float *__restrict__ w, __nv_bfloat16 *__r
     if (i < n) wb[i] = __float2bfloat16_rn(w[i]);
 }
 
-inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace
 
@@ -302,16 +333,15 @@ efie_status mlp_forward(efie_mlp *p, const float *X, int n) {
     const float *in = X;
     for (int l = 0; l < p->nl; l++) {
         const int fi = p->fin[l], fo = p->fout[l];
-        dim3 grid(cdiv(fo, BN), cdiv(n, BM), 1);
         const __nv_bfloat16 *W = p->wb.as<__nv_bfloat16>() + p->woff[l];
         const float *b = p->w.as<float>() + p->boff[l];
         // B(k, j) = W[j][k]
         if (l + 1 < p->nl)
-            k_mlp_gemm<__nv_bfloat16, EPI_FWD_HIDDEN><<<grid, GT, 0, s>>>(n, fo, fi, in, fi, 1, W, 1, fi, p->Z(l), fo, b,
-                                                                          p->A(l), nullptr, fi);
+            mlp_gemm<__nv_bfloat16, EPI_FWD_HIDDEN>(s, n, fo, fi, in, fi, 1, W, 1, fi, p->Z(l), fo, b, p->A(l), nullptr,
+                                                    fi);
         else
-            k_mlp_gemm<__nv_bfloat16, EPI_FWD_OUT><<<grid, GT, 0, s>>>(n, fo, fi, in, fi, 1, W, 1, fi, p->Z(l), fo, b,
-                                                                       nullptr, nullptr, fi);
+            mlp_gemm<__nv_bfloat16, EPI_FWD_OUT>(s, n, fo, fi, in, fi, 1, W, 1, fi, p->Z(l), fo, b, nullptr, nullptr,
+                                                 fi);
         EFIE_CUDA(cudaGetLastError());
         in = p->A(l);
     }
@@ -331,20 +361,18 @@ efie_status mlp_backward(efie_mlp *p, const float *X, const float *dY, int n) {
         // dW[o][i] += sum_m dz[m][o] ain[m][i]:  A(i=o, k=m) = dz[m*fo + o], B(k=m, j=i) = ain[m*fi + i]
         EFIE_CUDA(cudaEventRecord(p->ev_dz, s));
         EFIE_CUDA(cudaStreamWaitEvent(p->side, p->ev_dz, 0));
-        dim3 gw(cdiv(fi, BN), cdiv(fo, BM), cdiv(n, kchunk));
-        k_mlp_gemm<float, EPI_PARTIAL><<<gw, GT, 0, p->side>>>(fo, fi, n, dz, 1, fo, ain, fi, 1, p->gpart.as<float>(),
-                                                              fi, nullptr, nullptr, nullptr, kchunk);
+        mlp_gemm<float, EPI_PARTIAL>(p->side, fo, fi, n, dz, 1, fo, ain, fi, 1, p->gpart.as<float>(), fi, nullptr,
+                                     nullptr, nullptr, kchunk);
         const long cnt = (long)fo * fi;
-        k_sum_parts<<<(unsigned)((cnt + 255) / 256), 256, 0, p->side>>>((int)gw.z, cnt, p->gpart.as<float>(), gW);
+        k_sum_parts<<<(unsigned)((cnt + 255) / 256), 256, 0, p->side>>>(cdiv(n, kchunk), cnt, p->gpart.as<float>(), gW);
         k_colsum<<<dim3(cdiv(fo, 32), 1), 256, 0, p->side>>>(n, fo, dz, gb);
         EFIE_CUDA(cudaGetLastError());
         if (l > 0) {
             // dZ_{l-1}[m][i] = (sum_o dz[m][o] W[o][i]) * silu'(Z_{l-1}[m][i])
             float *out = p->dz.as<float>() + (size_t)p->cap * p->width * l;
             const __nv_bfloat16 *W = p->wb.as<__nv_bfloat16>() + p->woff[l];
-            dim3 gd(cdiv(fi, BN), cdiv(n, BM), 1);
-            k_mlp_gemm<__nv_bfloat16, EPI_BWD_DZ><<<gd, GT, 0, s>>>(n, fi, fo, dz, fo, 1, W, fi, 1, out, fi, nullptr,
-                                                                    nullptr, p->Z(l - 1), fo);
+            mlp_gemm<__nv_bfloat16, EPI_BWD_DZ>(s, n, fi, fo, dz, fo, 1, W, fi, 1, out, fi, nullptr, nullptr, p->Z(l - 1),
+                                                fo);
             EFIE_CUDA(cudaGetLastError());
             dz = out;
         }
