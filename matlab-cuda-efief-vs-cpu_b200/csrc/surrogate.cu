@@ -59,8 +59,7 @@ template <typename TB, int EPI, int T>
 __global__ void __launch_bounds__(GT, 4) k_mlp_gemm(int M, int N, int K, const float *__restrict__ A, long sai,
                                                  long sak, const TB *__restrict__ B, long sbk, long sbj,
                                                  float *__restrict__ C, int ldc, const float *__restrict__ bias,
-                                                 float *__restrict__ Aout, const float *__restrict__ Zprev,
-                                                 int kchunk) {
+                                                 float *__restrict__ Aout, int kchunk) {
     constexpr int R = T / 16, BK = T == 32 ? 32 : 16, PAD = R;   // PAD keeps the rows aligned for R floats
     __shared__ __align__(16) float As[BK][T + PAD];
     __shared__ __align__(16) float Bs[BK][T + PAD];
@@ -134,8 +133,8 @@ __global__ void __launch_bounds__(GT, 4) k_mlp_gemm(int M, int N, int K, const f
                 Aout[o] = z * sigm(z);
             } else if (EPI == EPI_FWD_OUT) {
                 C[o] = acc[a][b] + bias[j];
-            } else if (EPI == EPI_BWD_DZ) {
-                const float z = Zprev[o], s = sigm(z);
+            } else if (EPI == EPI_BWD_DZ) {   // in the place of Z
+                const float z = C[o], s = sigm(z);
                 C[o] = acc[a][b] * (s * (1.f + z * (1.f - s)));   // d silu / dz
             } else {
                 C[(long)blockIdx.z * M * ldc + o] = acc[a][b];
@@ -152,14 +151,14 @@ inline int cdiv(long a, long b) { return (int)((a + b - 1) / b); }
 constexpr long kLargeCtas = 148;
 template <typename TB, int EPI>
 void mlp_gemm(cudaStream_t s, int M, int N, int K, const float *A, long sai, long sak, const TB *B, long sbk, long sbj,
-              float *C, int ldc, const float *bias, float *Aout, const float *Zprev, int kchunk) {
+              float *C, int ldc, const float *bias, float *Aout, int kchunk) {
     const int nz = EPI == EPI_PARTIAL ? cdiv(K, kchunk) : 1;
     if ((long)cdiv(M, 64) * cdiv(N, 64) * nz >= kLargeCtas)
         k_mlp_gemm<TB, EPI, 64><<<dim3(cdiv(N, 64), cdiv(M, 64), nz), GT, 0, s>>>(M, N, K, A, sai, sak, B, sbk, sbj, C,
-                                                                                  ldc, bias, Aout, Zprev, kchunk);
+                                                                                  ldc, bias, Aout, kchunk);
     else
         k_mlp_gemm<TB, EPI, 32><<<dim3(cdiv(N, 32), cdiv(M, 32), nz), GT, 0, s>>>(M, N, K, A, sai, sak, B, sbk, sbj, C,
-                                                                                  ldc, bias, Aout, Zprev, kchunk);
+                                                                                  ldc, bias, Aout, kchunk);
 }
 
 // out[e] += sum_z part[z * count + e], z in order
@@ -272,8 +271,7 @@ struct efie_mlp {
     std::vector<size_t> woff, boff;              // offsets into the parameter vector
     size_t np = 0;
     DevBuf w, wb, g, m, v;                       // params FP32, BF16 copy, grads, Adam moments
-    DevBuf act;                                  // Z and A of every layer for `cap` rows
-    DevBuf dz;                                   // dZ of every hidden layer
+    DevBuf act;                                  // Z (backward: dZ) and A of every layer for `cap` rows
     // the weight gradients run beside the chain of dZ (fork and join by events,
     // also inside the captured step)
     cudaStream_t side = nullptr;
@@ -292,7 +290,7 @@ struct efie_mlp {
     float *A(int l) { return act.as<float>() + (size_t)cap * width * (2 * l + 1); }
     float *Y() { return Z(nl - 1); }
     std::vector<void *> step_ptrs() const {
-        return {w.p,  wb.p, g.p,  m.p,  v.p,  act.p, dz.p, gpart.p,
+        return {w.p,  wb.p, g.p,  m.p,  v.p,  act.p, gpart.p,
                 Xd.p, Td.p, perm.p, Xb.p, Tb.p, dY.p, step.p, hist.p};
     }
 
@@ -309,8 +307,8 @@ namespace {
 efie_status mlp_reserve(efie_mlp *p, int rows) {
     if (rows <= p->cap) return EFIE_OK;
     const int width = p->width;
+    p->cap = 0;   // a failed reservation leaves no buffers behind
     EFIE_TRY(p->act.reserve(sizeof(float) * (size_t)rows * width * 2 * p->nl));
-    EFIE_TRY(p->dz.reserve(sizeof(float) * (size_t)rows * width * p->nl));
     if (!p->side) {
         EFIE_CUDA(cudaStreamCreateWithFlags(&p->side, cudaStreamNonBlocking));
         for (cudaEvent_t *e : {&p->ev_dz, &p->ev_side})
@@ -337,11 +335,9 @@ efie_status mlp_forward(efie_mlp *p, const float *X, int n) {
         const float *b = p->w.as<float>() + p->boff[l];
         // B(k, j) = W[j][k]
         if (l + 1 < p->nl)
-            mlp_gemm<__nv_bfloat16, EPI_FWD_HIDDEN>(s, n, fo, fi, in, fi, 1, W, 1, fi, p->Z(l), fo, b, p->A(l), nullptr,
-                                                    fi);
+            mlp_gemm<__nv_bfloat16, EPI_FWD_HIDDEN>(s, n, fo, fi, in, fi, 1, W, 1, fi, p->Z(l), fo, b, p->A(l), fi);
         else
-            mlp_gemm<__nv_bfloat16, EPI_FWD_OUT>(s, n, fo, fi, in, fi, 1, W, 1, fi, p->Z(l), fo, b, nullptr, nullptr,
-                                                 fi);
+            mlp_gemm<__nv_bfloat16, EPI_FWD_OUT>(s, n, fo, fi, in, fi, 1, W, 1, fi, p->Z(l), fo, b, nullptr, fi);
         EFIE_CUDA(cudaGetLastError());
         in = p->A(l);
     }
@@ -362,17 +358,16 @@ efie_status mlp_backward(efie_mlp *p, const float *X, const float *dY, int n) {
         EFIE_CUDA(cudaEventRecord(p->ev_dz, s));
         EFIE_CUDA(cudaStreamWaitEvent(p->side, p->ev_dz, 0));
         mlp_gemm<float, EPI_PARTIAL>(p->side, fo, fi, n, dz, 1, fo, ain, fi, 1, p->gpart.as<float>(), fi, nullptr,
-                                     nullptr, nullptr, kchunk);
+                                     nullptr, kchunk);
         const long cnt = (long)fo * fi;
         k_sum_parts<<<(unsigned)((cnt + 255) / 256), 256, 0, p->side>>>(cdiv(n, kchunk), cnt, p->gpart.as<float>(), gW);
         k_colsum<<<dim3(cdiv(fo, 32), 1), 256, 0, p->side>>>(n, fo, dz, gb);
         EFIE_CUDA(cudaGetLastError());
         if (l > 0) {
             // dZ_{l-1}[m][i] = (sum_o dz[m][o] W[o][i]) * silu'(Z_{l-1}[m][i])
-            float *out = p->dz.as<float>() + (size_t)p->cap * p->width * l;
+            float *out = p->Z(l - 1);   // not read again
             const __nv_bfloat16 *W = p->wb.as<__nv_bfloat16>() + p->woff[l];
-            mlp_gemm<__nv_bfloat16, EPI_BWD_DZ>(s, n, fi, fo, dz, fo, 1, W, fi, 1, out, fi, nullptr, nullptr, p->Z(l - 1),
-                                                fo);
+            mlp_gemm<__nv_bfloat16, EPI_BWD_DZ>(s, n, fi, fo, dz, fo, 1, W, fi, 1, out, fi, nullptr, nullptr, fo);
             EFIE_CUDA(cudaGetLastError());
             dz = out;
         }

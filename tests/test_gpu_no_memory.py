@@ -59,3 +59,21 @@ def test_sweep_without_room_for_moments(problem, limit):
     assert np.max(np.abs(again - short) / np.abs(short)) <= 1e-6
     assert np.max(np.abs(last - short) / np.abs(short)) <= 1e-6
     assert np.max(np.abs(Zm - Zp) / np.abs(Zm)) <= 1e-6   # the sweeps' bound on both
+
+
+def test_network_after_a_batch_without_room(limit):
+    m = pkg()
+    sur = importlib.import_module(m.__name__ + ".surrogate")
+    net = sur.Surrogate(n_hidden=256, n_layers=4, seed=1)
+    r = np.random.default_rng(2)
+    X, T = r.uniform(-1, 1, (60000, 5)).astype(np.float32), r.uniform(-1, 1, (60000, 3)).astype(np.float32)
+    Y, (loss, grad) = net.forward(X[:100]), net.loss_grad(X[:100], T[:100])
+    limit(100 * MB)   # 60000 rows of activations: 614 MB
+    with pytest.raises(m.MexError) as e:
+        net.loss_grad(X, T)
+    assert e.value.identifier == "efie:nomem"
+    assert np.array_equal(net.forward(X[:100]), Y)
+    limit(0)
+    loss2, grad2 = net.loss_grad(X[:100], T[:100])
+    assert loss2 == loss and np.array_equal(grad2, grad)
+    assert np.isfinite(net.loss_grad(X, T)[0])
