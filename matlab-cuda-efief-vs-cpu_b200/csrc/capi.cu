@@ -383,8 +383,12 @@ efie_status copy_to_host(efie_ctx *ctx, void *dst, const void *src, size_t bytes
     const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
     const int nt = (int)std::min(12u, std::thread::hardware_concurrency() * 3 / 4);
-    HostCopy hc;
     bool ok = bytes >= kCopyMin && pageable && nt > 1;
+    // callers on other threads of the context wait for the staging buffers, as
+    // they would for the stream; given up after hc has joined the threads
+    std::unique_lock<std::mutex> lk(ctx->pinned_mu, std::defer_lock);
+    if (ok) lk.lock();
+    HostCopy hc;
     if (ok && !ctx->pinned && cudaHostAlloc(&ctx->pinned, kPiece * kCopyBufs, cudaHostAllocDefault) != cudaSuccess) {
         ctx->pinned = nullptr;
         ok = false;
@@ -419,6 +423,7 @@ efie_status copy_to_host(efie_ctx *ctx, void *dst, const void *src, size_t bytes
         }
     }
     if (!ok) {
+        if (lk.owns_lock()) lk.unlock();
         cudaGetLastError();
         EFIE_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s));
         EFIE_CUDA(cudaStreamSynchronize(s));

@@ -3,6 +3,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <mutex>
 #include <string>
 
 #include "../../include/efie_b200.h"
@@ -146,6 +147,7 @@ struct efie_ctx {
     int num_sms = 0;
     int cc_major = 0;
     void *pinned = nullptr;   // staging of large results to pageable host memory (copy_to_host)
+    std::mutex pinned_mu;     // held while a result passes through it
     DevBuf status;   // device-side error flags of bounded waits (int32[8])
     KernelLog log;
 };
