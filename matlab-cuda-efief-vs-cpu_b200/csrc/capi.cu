@@ -11,6 +11,8 @@
 #include <mutex>
 #include <vector>
 
+#include <sys/mman.h>
+
 #include "efie_internal.h"
 #include "solve.h"
 
@@ -121,7 +123,7 @@ extern "C" void efie_ctx_destroy(efie_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->solver) cusolverDnDestroy(ctx->solver);
     ctx->status.release();
-    if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    ctx->stage.release();
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
     efie_pool_trim(ctx->device);
     delete ctx;
@@ -358,23 +360,81 @@ namespace {
 // 3086, 152 MB: 35 ms, 4.3 GB/s).  Here pieces of 2 MB -- on the destination's
 // 2 MB boundaries, so that no two threads fault on one huge page -- land in
 // pinned buffers while several threads copy the ones before out, a whole piece
-// each.  The pinned buffers (48 MB; allocating them takes 45 ms) stay with the
-// context, the threads end with the call; small results, pinned destinations
+// each.  The threads end with the call; small results, pinned destinations
 // and any failure to set up take the plain copy.
+//
+// The pinned pieces stay with the context, a third of the largest result so
+// far and at most 48 MB.  They are huge pages that several threads touch and
+// one call then registers: a context's first result of Ne 3086 takes 9.4 ms
+// (later ones 5.2), by the plain copy 34.7, and with cudaHostAlloc, which
+// needs 25 to 45 ms for 48 MB, it took 42.
 constexpr size_t kPiece = (size_t)2 << 20;
 constexpr int kCopyBufs = 24;
 constexpr size_t kCopyMin = (size_t)8 << 20;   // below it the threads cost more than they save
 
-struct HostCopy {
-    cudaEvent_t ev[kCopyBufs] = {};
+struct Joined {
     std::vector<std::thread> threads;
+    ~Joined() {
+        for (std::thread &t : threads) t.join();
+    }
+};
+
+}  // namespace
+
+void HostStage::grow(size_t n) {
+    n = std::min<size_t>(n, kCopyBufs);
+    if (n <= pieces.size()) return;
+    n -= pieces.size();
+    const size_t bytes = n * kPiece, len = bytes + kPiece;
+    void *p = mmap(nullptr, len, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (p == MAP_FAILED) return;
+    char *base = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) + kPiece - 1) / kPiece * kPiece);
+    madvise(base, bytes, MADV_HUGEPAGE);
+    try {
+        pieces.reserve(pieces.size() + n);
+        maps.reserve(maps.size() + 1);
+        Joined touch;
+        const size_t nt = std::min<size_t>(n, 8);
+        for (size_t t = 0; t < nt; t++)
+            touch.threads.emplace_back([=] {
+                for (size_t i = t; i < n; i += nt)
+                    for (size_t o = 0; o < kPiece; o += 4096) base[i * kPiece + o] = 0;
+            });
+    } catch (...) {   // no memory or no threads to be had
+        munmap(p, len);
+        return;
+    }
+    if (cudaHostRegister(base, bytes, cudaHostRegisterDefault) != cudaSuccess) {
+        cudaGetLastError();
+        munmap(p, len);
+        return;
+    }
+    maps.push_back(Map{p, len, base});
+    for (size_t i = 0; i < n; i++) pieces.push_back(base + i * kPiece);
+}
+
+void HostStage::release() {
+    for (const Map &m : maps) {
+        cudaHostUnregister(m.base);
+        munmap(m.p, m.len);
+    }
+    maps.clear();
+    pieces.clear();
+}
+
+namespace {
+
+struct HostCopy {
+    struct Events {
+        cudaEvent_t ev[kCopyBufs] = {};
+        ~Events() {
+            for (cudaEvent_t e : ev)
+                if (e) cudaEventDestroy(e);
+        }
+    } events;
     std::atomic<int64_t> ready{0};             // pieces in their pinned buffers (-1: stop)
     std::atomic<int64_t> out[kCopyBufs];       // the last piece copied out of each buffer
-    ~HostCopy() {
-        for (std::thread &t : threads) t.join();
-        for (cudaEvent_t e : ev)
-            if (e) cudaEventDestroy(e);
-    }
+    Joined copiers;                            // joined first
 };
 
 efie_status copy_to_host(efie_ctx *ctx, void *dst, const void *src, size_t bytes) {
@@ -382,21 +442,21 @@ efie_status copy_to_host(efie_ctx *ctx, void *dst, const void *src, size_t bytes
     cudaPointerAttributes at{};
     const bool pageable = cudaPointerGetAttributes(&at, dst) != cudaSuccess || at.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
-    const int nt = (int)std::min(12u, std::thread::hardware_concurrency() * 3 / 4);
+    int nt = (int)std::min(12u, std::thread::hardware_concurrency() * 3 / 4);
     bool ok = bytes >= kCopyMin && pageable && nt > 1;
     // callers on other threads of the context wait for the staging buffers, as
     // they would for the stream; given up after hc has joined the threads
-    std::unique_lock<std::mutex> lk(ctx->pinned_mu, std::defer_lock);
+    std::unique_lock<std::mutex> lk(ctx->stage.mu, std::defer_lock);
     if (ok) lk.lock();
     HostCopy hc;
-    if (ok && !ctx->pinned && cudaHostAlloc(&ctx->pinned, kPiece * kCopyBufs, cudaHostAllocDefault) != cudaSuccess) {
-        ctx->pinned = nullptr;
-        ok = false;
-    }
-    char *const pinned = static_cast<char *>(ctx->pinned);
-    for (int b = 0; ok && b < kCopyBufs; b++) {
-        ok = cudaEventCreateWithFlags(&hc.ev[b], cudaEventDisableTiming) == cudaSuccess;
-        hc.out[b].store(b - kCopyBufs);
+    if (ok) ctx->stage.grow(bytes / (3 * kPiece) + 1);
+    const std::vector<char *> &piece = ctx->stage.pieces;
+    const int nbuf = ok ? (int)piece.size() : 0;
+    nt = std::min(nt, nbuf);
+    ok = ok && nt > 1;
+    for (int b = 0; ok && b < nbuf; b++) {
+        ok = cudaEventCreateWithFlags(&hc.events.ev[b], cudaEventDisableTiming) == cudaSuccess;
+        hc.out[b].store(b - nbuf);
     }
     // piece i covers [begin(i), begin(i + 1)) of the result
     const size_t head = (kPiece - reinterpret_cast<uintptr_t>(dst) % kPiece) % kPiece;
@@ -407,14 +467,14 @@ efie_status copy_to_host(efie_ctx *ctx, void *dst, const void *src, size_t bytes
     if (ok) {
         try {
             for (int t = 0; t < nt; t++)
-                hc.threads.emplace_back([&hc, begin, pinned, t, nt, n, dst] {
+                hc.copiers.threads.emplace_back([&hc, &piece, begin, t, nt, n, nbuf, dst] {
                     for (int64_t i = t; i < n; i += nt) {
                         int64_t r;
                         while ((r = hc.ready.load(std::memory_order_acquire)) >= 0 && r <= i) std::this_thread::yield();
                         if (r < 0) return;
                         const size_t off = begin(i);
-                        std::memcpy(static_cast<char *>(dst) + off, pinned + (i % kCopyBufs) * kPiece, begin(i + 1) - off);
-                        hc.out[i % kCopyBufs].store(i, std::memory_order_release);
+                        std::memcpy(static_cast<char *>(dst) + off, piece[i % nbuf], begin(i + 1) - off);
+                        hc.out[i % nbuf].store(i, std::memory_order_release);
                     }
                 });
         } catch (...) {   // no threads to be had
@@ -434,16 +494,16 @@ efie_status copy_to_host(efie_ctx *ctx, void *dst, const void *src, size_t bytes
     while (handed < n && e == cudaSuccess) {
         // fetch while buffers are free (their previous piece is out), then hand over the oldest in flight
         while (fetched < n && e == cudaSuccess &&
-               hc.out[fetched % kCopyBufs].load(std::memory_order_acquire) == fetched - kCopyBufs) {
-            const int b = (int)(fetched % kCopyBufs);
+               hc.out[fetched % nbuf].load(std::memory_order_acquire) == fetched - nbuf) {
+            const int b = (int)(fetched % nbuf);
             const size_t off = begin(fetched);
-            e = cudaMemcpyAsync(pinned + b * kPiece, static_cast<const char *>(src) + off, begin(fetched + 1) - off,
+            e = cudaMemcpyAsync(piece[b], static_cast<const char *>(src) + off, begin(fetched + 1) - off,
                                 cudaMemcpyDeviceToHost, s);
-            if (e == cudaSuccess) e = cudaEventRecord(hc.ev[b], s);
+            if (e == cudaSuccess) e = cudaEventRecord(hc.events.ev[b], s);
             fetched++;
         }
         if (handed < fetched && e == cudaSuccess) {
-            e = cudaEventSynchronize(hc.ev[handed % kCopyBufs]);
+            e = cudaEventSynchronize(hc.events.ev[handed % nbuf]);
             if (e == cudaSuccess) hc.ready.store(++handed, std::memory_order_release);
         } else {
             std::this_thread::yield();
@@ -454,7 +514,7 @@ efie_status copy_to_host(efie_ctx *ctx, void *dst, const void *src, size_t bytes
         cudaStreamSynchronize(s);   // copies in flight write the pinned buffers
         return efie_fail(EFIE_ERR_CUDA, std::string("copy to host: ") + cudaGetErrorString(e));
     }
-    return EFIE_OK;   // ~HostCopy joins the threads
+    return EFIE_OK;   // hc joins the threads
 }
 
 }  // namespace

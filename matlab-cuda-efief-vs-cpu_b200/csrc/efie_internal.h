@@ -139,6 +139,16 @@ struct KernelLog {
     }
 };
 
+// Pinned host pieces of 2 MB, as many as the results so far asked for.
+struct HostStage {
+    struct Map { void *p; size_t len; void *base; };   // an anonymous mapping and its registered part
+    std::mutex mu;                                      // held while a result passes through
+    std::vector<char *> pieces;
+    std::vector<Map> maps;
+    void grow(size_t n);   // towards n pieces: fewer when the memory cannot be had
+    void release();
+};
+
 struct efie_ctx {
     int device = 0;
     cudaStream_t own_stream = nullptr;
@@ -146,8 +156,7 @@ struct efie_ctx {
     cusolverDnHandle_t solver = nullptr;
     int num_sms = 0;
     int cc_major = 0;
-    void *pinned = nullptr;   // staging of large results to pageable host memory (copy_to_host)
-    std::mutex pinned_mu;     // held while a result passes through it
+    HostStage stage;          // large results to pageable host memory (copy_to_host)
     DevBuf status;   // device-side error flags of bounded waits (int32[8])
     KernelLog log;
 };
