@@ -1095,19 +1095,20 @@ efie_status efie_geom_upload(efie_ctx *ctx, const efie_mesh *mesh, const efie_pr
         std::vector<std::vector<int>> vt(Nv);
         for (int t = 0; t < Nt; t++)
             for (int j = 0; j < 3; j++) vt[mesh->F[t + (size_t)j * Nt] - 1].push_back(t);
-        std::vector<int> seen(Nt, -1);
-        for (int t1 = 0; t1 < Nt; t1++) {
+        // a column t2 at a time, its t1 rising: ordered by (t2, t1) like the near list
+        std::vector<int> seen(Nt, -1), col;
+        for (int t2 = 0; t2 < Nt; t2++) {
+            col.clear();
             for (int j = 0; j < 3; j++)
-                for (int t2 : vt[mesh->F[t1 + (size_t)j * Nt] - 1])
-                    if (t2 >= t1 && seen[t2] != t1) {
-                        seen[t2] = t1;
-                        list.push_back(make_int2(t1, t2));
-                    }
+                for (int t1 : vt[mesh->F[t2 + (size_t)j * Nt] - 1]) {   // rising
+                    if (t1 > t2) break;
+                    if (seen[t1] == t2) continue;
+                    seen[t1] = t2;
+                    col.push_back(t1);
+                }
+            std::sort(col.begin(), col.end());
+            for (int t1 : col) list.push_back(make_int2(t1, t2));
         }
-        // ordered by (t2, t1) like the near list
-        std::sort(list.begin(), list.end(), [](const int2 &a, const int2 &b) {
-            return a.y != b.y ? a.y < b.y : a.x < b.x;
-        });
         g.symmetric = true;
         g.n_adj = (int)list.size();
         g.n_near = 0;
