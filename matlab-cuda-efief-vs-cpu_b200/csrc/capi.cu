@@ -1385,9 +1385,12 @@ struct CentroidPack {
 };
 
 // false where the rule does not fit a prepack: an RWG side whose area is not
-// its triangle's (to rounding), or both sides on one triangle
+// its triangle's (to rounding), both sides on one triangle, or so many
+// triangles without basis functions that the plan's mask of triangle pairs
+// would outgrow the matrix (Nt^2 bytes against 16 Ne^2)
 bool centroid_pack(const efie_mesh *m, double self_alpha, CentroidPack &c) {
     const int Nt = m->Nt, Nv = m->Nv;
+    if (Nt > 4 * (int64_t)m->Ne) return false;
     c.r.resize(3 * (size_t)Nt);
     c.w.resize(Nt);
     c.a.resize(Nt);

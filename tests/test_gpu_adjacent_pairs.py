@@ -1,6 +1,6 @@
 """The extraction scheme on meshes whose triangles come in any order: the
 adjacent pairs are found and ordered whatever the numbering, so the series'
-matrices match the oracle's, and a plan's creation does not sort them."""
+matrices match the oracle's."""
 import ctypes as C
 import importlib
 
