@@ -15,6 +15,10 @@ import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 REF_DIR = os.path.join(HERE, "_ref")
+# the reference's source of each library (oracle/Makefile)
+SOURCES = {"ggassemble_ref": "ggassemble_ZV_EFIE_RWG_DIFF_GPU_FAST.cu",
+           "gassemble_ref": "gassemble_ZV_EFIE_RWG_DIFF_GPU_FAST.cu",
+           "patch_sweep_fastquad_ref": "patch_sweep_fastquad_cuda.cu", "patch_sweep_cuda_ref": "patch_sweep_cuda.cu"}
 MX_DOUBLE, MX_INT32, MX_UINT8 = 6, 12, 9
 
 
@@ -25,14 +29,21 @@ class RefError(RuntimeError):
 
 
 class RefMissing(FileNotFoundError, unittest.SkipTest):
-    """The reference's sources were not there to build: a comparison with it is skipped."""
+    """The reference's sources are not there to build: a comparison with it is skipped."""
+
+
+def missing(name, path):
+    """The error for a library that is not built: a skip only without its source."""
+    src = os.path.join(os.environ.get("EFIE_REFERENCE_DIR", "/root/reference"), SOURCES[name])
+    what = path + " (build with: make -C oracle)"
+    return FileNotFoundError(what) if os.path.exists(src) else RefMissing(what)
 
 
 class RefMex:
     def __init__(self, name):
         path = os.path.join(REF_DIR, name + ".so")
         if not os.path.exists(path):
-            raise RefMissing(path + " (build with: make -C oracle)")
+            raise missing(name, path)
         L = C.CDLL(path)
         L.fm_numeric.restype = C.c_void_p
         L.fm_numeric.argtypes = [C.c_int, C.c_int, C.POINTER(C.c_size_t), C.c_void_p, C.c_void_p]
