@@ -432,6 +432,12 @@ efie_status efie_debug_plan_series(efie_plan *plan, const double *freqs, int32_t
  * blocks are read.  No counterpart in the reference. */
 efie_status efie_debug_snapshot_guess(efie_ctx *ctx, int32_t N, int32_t k, const efie_c128 *Z, const efie_c128 *xs,
                                       const efie_c128 *b, efie_c128 *x);
+/* The same for nf matrices Z[nf][N x N] at once, as a batch of frequencies:
+ * matrix f combines the k[f] vectors xs[pos[f][0 .. k[f] - 1]] (pos [nf][23],
+ * xs [nx][N]) into x[f][N]. */
+efie_status efie_debug_snapshot_guesses(efie_ctx *ctx, int32_t N, int32_t nf, int32_t nx, const int32_t *k,
+                                        const int32_t *pos, const efie_c128 *Z, const efie_c128 *xs,
+                                        const efie_c128 *b, efie_c128 *x);
 
 /* ---------------------------------------------------------------------- */
 /* Centroid assembly without device allocation                             */

@@ -136,6 +136,7 @@ SIGNATURES = {
     "efie_debug_limit_allocations": (None, [C.c_size_t]),
     "efie_debug_plan_series": (C.c_int, [_P, c_double_p, C.c_int32, C.c_int32, c_int32_p, _P]),
     "efie_debug_snapshot_guess": (C.c_int, [_P, C.c_int32, C.c_int32, _P, _P, _P, _P]),
+    "efie_debug_snapshot_guesses": (C.c_int, [_P, C.c_int32, C.c_int32, C.c_int32, _P, _P, _P, _P, _P, _P]),
     "efie_debug_set_wait_test": (C.c_int, [C.c_int32, C.c_int64]),
     "efie_gassemble_zv_noalloc": (C.c_int, [C.c_int, _P, C.c_int32, C.c_int32, C.c_int32] + [_P] * 12 +
                                   [c128, C.c_double, C.c_double, c128, c_double_p, _P, _P]),

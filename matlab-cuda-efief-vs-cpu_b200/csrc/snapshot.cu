@@ -402,35 +402,53 @@ efie_status efie_snapshot_guess(efie_ctx *ctx, SolveWork &w, const void *Z, size
     return EFIE_OK;
 }
 
-// Test entry: one guess from host arrays (Z column-major N x N, xs [k][N]).
-extern "C" efie_status efie_debug_snapshot_guess(efie_ctx *ctx, int32_t N, int32_t k, const efie_c128 *Z,
-                                                 const efie_c128 *xs, const efie_c128 *b, efie_c128 *x) {
-    if (!ctx || N < 1 || k < 1 || k > KMAX || !Z || !xs || !b || !x)
-        return efie_fail(EFIE_ERR_ARGS, "efie_debug_snapshot_guess: bad arguments");
+// Test entries: guesses from host arrays (Z column-major N x N, xs [nx][N]).
+extern "C" efie_status efie_debug_snapshot_guesses(efie_ctx *ctx, int32_t N, int32_t nf, int32_t nx, const int32_t *k,
+                                                   const int32_t *pos, const efie_c128 *Z, const efie_c128 *xs,
+                                                   const efie_c128 *b, efie_c128 *x) {
+    if (!ctx || N < 1 || nf < 1 || nf > EFIE_MAX_BATCH || nx < 1 || !k || !pos || !Z || !xs || !b || !x)
+        return efie_fail(EFIE_ERR_ARGS, "efie_debug_snapshot_guesses: bad arguments");
+    SnapSpec sp{};
+    for (int f = 0; f < nf; f++) {
+        sp.k[f] = k[f];
+        bool ok = k[f] >= 1 && k[f] <= KMAX;
+        for (int j = 0; ok && j < k[f]; j++) {
+            sp.pos[f][j] = pos[f * KMAX + j];
+            ok = sp.pos[f][j] >= 0 && sp.pos[f][j] < nx;
+        }
+        if (!ok) return efie_fail(EFIE_ERR_ARGS, "efie_debug_snapshot_guesses: bad snapshot list");
+    }
     DeviceGuard dg(ctx->device);
     ctx->log.reset(false);
     cudaStream_t s = ctx->stream;
     SolveWork w;
     w.N = N;
-    w.B = 1;
-    EFIE_TRY(w.ctl.reserve(64));
-    EFIE_CUDA(cudaMemsetAsync(w.ctl.p, 0, 64, s));
+    w.B = nf;
+    EFIE_TRY(w.ctl.reserve(64 * (size_t)nf));
+    EFIE_CUDA(cudaMemsetAsync(w.ctl.p, 0, 64 * (size_t)nf, s));
     DevBuf dZ, dx, db, dg0;
     const size_t v = sizeof(efie_c128) * (size_t)N;
-    EFIE_TRY(dZ.reserve(v * N));
-    EFIE_TRY(dx.reserve(v * k));
+    EFIE_TRY(dZ.reserve(v * N * nf));
+    EFIE_TRY(dx.reserve(v * nx));
     EFIE_TRY(db.reserve(v));
-    EFIE_TRY(dg0.reserve(v));
-    EFIE_CUDA(cudaMemcpyAsync(dZ.p, Z, v * N, cudaMemcpyHostToDevice, s));
-    EFIE_CUDA(cudaMemcpyAsync(dx.p, xs, v * k, cudaMemcpyHostToDevice, s));
+    EFIE_TRY(dg0.reserve(v * nf));
+    EFIE_CUDA(cudaMemcpyAsync(dZ.p, Z, v * N * nf, cudaMemcpyHostToDevice, s));
+    EFIE_CUDA(cudaMemcpyAsync(dx.p, xs, v * nx, cudaMemcpyHostToDevice, s));
     EFIE_CUDA(cudaMemcpyAsync(db.p, b, v, cudaMemcpyHostToDevice, s));
-    SnapSpec sp{};
-    sp.k[0] = k;
-    for (int j = 0; j < k; j++) sp.pos[0][j] = j;
-    EFIE_TRY(efie_snapshot_guess(ctx, w, dZ.p, (size_t)N * N, dx.p, db.p, 1, sp, dg0.p));
-    int err = 0;
-    EFIE_CUDA(cudaMemcpyAsync(&err, w.ctl.as<char>() + 36, sizeof(int), cudaMemcpyDeviceToHost, s));
-    EFIE_CUDA(cudaMemcpyAsync(x, dg0.p, v, cudaMemcpyDeviceToHost, s));
+    EFIE_TRY(efie_snapshot_guess(ctx, w, dZ.p, (size_t)N * N, dx.p, db.p, nf, sp, dg0.p));
+    std::vector<char> ctl(64 * (size_t)nf);
+    EFIE_CUDA(cudaMemcpyAsync(ctl.data(), w.ctl.p, ctl.size(), cudaMemcpyDeviceToHost, s));
+    EFIE_CUDA(cudaMemcpyAsync(x, dg0.p, v * nf, cudaMemcpyDeviceToHost, s));
     EFIE_CUDA(cudaStreamSynchronize(s));
-    return err ? efie_fail(EFIE_ERR_TIMEOUT, "efie_debug_snapshot_guess: device error flag") : EFIE_OK;
+    for (int f = 0; f < nf; f++)
+        if (*reinterpret_cast<const int *>(ctl.data() + 64 * f + 36))
+            return efie_fail(EFIE_ERR_TIMEOUT, "efie_debug_snapshot_guesses: device error flag");
+    return EFIE_OK;
+}
+
+extern "C" efie_status efie_debug_snapshot_guess(efie_ctx *ctx, int32_t N, int32_t k, const efie_c128 *Z,
+                                                 const efie_c128 *xs, const efie_c128 *b, efie_c128 *x) {
+    int32_t pos[KMAX];
+    for (int j = 0; j < KMAX; j++) pos[j] = j;
+    return efie_debug_snapshot_guesses(ctx, N, 1, k, &k, pos, Z, xs, b, x);
 }
