@@ -240,7 +240,11 @@ def roofline(classes, name=None, fp64_peak=None):
     else:
         achieved = per_launch_work / (per_launch_ms * 1e-3) / 1e9
         peak = peaks["hbm_gbs"]
-        out = dict(bound="hbm", unit="GB/s", peak_source=src)
+        # the products class holds both kinds: one vector a product (bound by
+        # HBM) and the starts' products with up to 16 (bound by FP64); the
+        # rate is that of the bytes of Z either way
+        out = dict(bound="hbm" if name != "residual" else "hbm (one vector), fp64 (several vectors)", unit="GB/s",
+                   peak_source=src)
     out.update(kernel=name, achieved=achieved, peak=peak,
                frac=(achieved / peak) if (peak and achieved is not None) else None,
                traffic=tr, launches=c["launches"], ms_per_launch=per_launch_ms)
@@ -568,7 +572,7 @@ def run_ours(args):
                     roofline=roofline(classes),
                     roofline_assembly=roofline(classes, "quad", fp64_peak),
                     roofline_tensor=roofline(classes, "gemm"),
-                    # the HBM-bound classes: algorithmic bytes over their event time
+                    # algorithmic bytes over their event time
                     roofline_hbm={k: roofline(classes, k) for k in ("trsv", "residual", "gather")},
                     phases_ms_per_point={k: v["ms"] / B for k, v in classes.items()},
                     phases_note="one extra step with per-launch CUDA events (eager launches, the LU's "
