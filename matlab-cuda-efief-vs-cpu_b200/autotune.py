@@ -63,13 +63,16 @@ def tuned_opts(Ne, sms=None):
 def _time(plan_args, freqs, repeats, **kw):
     from .api import SweepPlan, sweep_opts
     from . import _native
-    try:
+    plan = None
+    try:   # a sweep reserves memory too: its matrices' moments or pair values, and GMRES's vectors
         plan = SweepPlan(*plan_args, opts=sweep_opts(nfreq_hint=len(freqs), **kw))
+        plan.run(freqs)                              # warm-up: workspaces, kernels, graph
     except _native.MexError as e:
+        if plan is not None:
+            plan.close()
         if e.identifier != "efie:nomem":
             raise
         return len(plan_args[2]), None   # a batch too large for this GPU: no candidate
-    plan.run(freqs)                                  # warm-up: workspaces, kernels, graph
     t0 = time.perf_counter()
     ok = True
     for _ in range(repeats):
