@@ -1000,16 +1000,18 @@ static bool snapshot_nodes(const int *pos, int nb, const std::vector<double> &fs
     return true;
 }
 
-// What a sweep on shared factors solves to, as a part of the residual target
-// (efie_mixed_gmres: aim).  The frequencies of its first batch become the snapshots
-// every later start is a combination of, so their errors enter all of them;
-// the others end on a neighbour's factors, or on no step at all, and such a
-// residual of half the target leaves more error in the currents than one
-// that the frequency's own factors have brought there.  Measured against the
-// complex128 solver (37 sweeps, Ne 500 to 20000; the worst and the median
-// current errors, geometric means over them): 1.45 and 1.58 times those of
-// interpolated starts at half the target for all, 0.51 and 0.78 times with
+// What a sweep that may share factors solves to, as a part of the residual
+// target (efie_mixed_gmres: aim).  The frequencies of its first batch become
+// the snapshots every later start is a combination of, so their errors enter
+// all of them; the others end on a neighbour's factors, or on no step at all,
+// and such a residual of half the target leaves more error in the currents
+// than one that the frequency's own factors have brought there.  Measured
+// against the complex128 solver (37 sweeps, Ne 500 to 20000; the worst and the
+// median current errors, geometric means over them): 1.45 and 1.58 times those
+// of interpolated starts at half the target for all, 0.51 and 0.78 times with
 // these; it costs 3 % of the time (Ne 6968, 101 frequencies: 86.5 -> 95 ms).
+// Sweeps short enough for one batch: medians 1.7 times (Ne 2404 and 4110)
+// those of two batches at half the target, 0.6 to 1.02 with a tenth.
 constexpr double kAimSnapshots = 0.02, kAimShared = 0.1, kAim = 0.5;
 
 static bool g_warm_start_disabled = false;
@@ -1240,7 +1242,9 @@ extern "C" efie_status efie_plan_run(efie_plan *p, const double *freqs, int32_t 
             else
                 rc = efie_mixed_gmres(ctx, p->sw, p->Z.p, NN, p->b.p, p->x.p, p->bnorm, p->opts.refine_tol,
                                       p->opts.refine_max_iter, active, &rr, guess,
-                                      !share ? kAim : bi == 0 ? kAimSnapshots : kAimShared);
+                                      !share && !(anchored && Nf > 1) ? kAim
+                                      : share && bi == 0              ? kAimSnapshots
+                                                                      : kAimShared);
             if (rc != EFIE_OK) break;
             S->refine_iters_max = std::max(S->refine_iters_max, rr.iters);
             int err1[EFIE_MAX_BATCH];   // device error codes of the first attempt

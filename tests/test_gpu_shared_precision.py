@@ -35,3 +35,16 @@ def test_shared_sweep_meets_the_complex128_solver(pitch, nf):
     # (measured with every frequency factored: 3.0e-11 residual, 3.6e-11 to 1.4e-10 error)
     assert np.max(np.abs(Zin - Zr) / np.abs(Zr)) <= TOL
     assert np.max(np.linalg.norm(I - Ir, axis=0) / np.linalg.norm(Ir, axis=0)) <= 1.5 * TOL
+
+
+@pytest.mark.parametrize("nf", [8, 15])
+def test_sweep_of_one_batch_aims_below_half_the_target(nf):
+    sur, d = _design(2e-3)
+    plan = sur.design_plan(d, nfreq=nf)
+    for freqs in (d.band(nf), d.band(nf)[:1]):
+        plan.run(freqs)
+        st = plan.stats
+        assert st["n_shared_factors"] == 0   # all factored together
+        # a single frequency has no neighbour to be compared with: half the target, as ever
+        assert st["max_relres"] <= (0.1 * TOL + 5e-12 if len(freqs) > 1 else TOL)
+    plan.close()
