@@ -195,7 +195,9 @@ typedef struct efie_sweep_opts {
                                 size gives a sweep at least g batches.  1: every
                                 frequency is factored.  0 (default): automatic, a
                                 first batch of 3 to 24 frequencies (48000 / Ne, at
-                                most what the band needs) is factored for all */
+                                most what the band needs) is factored for all; a
+                                batch that cannot hold them: groups with
+                                g = Ne / 1200 within [2, 8] */
 } efie_sweep_opts;
 
 /* Fill `o` with the defaults listed above. */

@@ -1006,10 +1006,11 @@ static bool snapshot_nodes(const int *pos, int nb, const std::vector<double> &fs
 // all of them; the others end on a neighbour's factors, or on no step at all,
 // and such a residual of half the target leaves more error in the currents
 // than one that the frequency's own factors have brought there.  Measured
-// against the complex128 solver (37 sweeps, Ne 500 to 20000; the worst and the
+// against the complex128 solver (38 sweeps, Ne 500 to 20000; the worst and the
 // median current errors, geometric means over them): 1.45 and 1.58 times those
 // of interpolated starts at half the target for all, 0.51 and 0.78 times with
-// these; it costs 3 % of the time (Ne 6968, 101 frequencies: 86.5 -> 95 ms).
+// these; it costs 3 % of the time (Ne 6968, 101 frequencies: 86.5 -> 95 ms;
+// starts accepted at a quarter of the target: 0.52 and 0.81 times, 92 ms).
 // Sweeps short enough for one batch: medians 1.7 times (Ne 2404 and 4110)
 // those of two batches at half the target, 0.6 to 1.02 with a tenth.
 constexpr double kAimSnapshots = 0.02, kAimShared = 0.1, kAim = 0.5;
@@ -1447,9 +1448,10 @@ extern "C" efie_status efie_patch_sweep_centroid(efie_ctx *ctx, const efie_mesh 
     o.port_model = EFIE_PORT_EDGE_DIFF;
     // The one-point rule as a prepack: the centroid with the area as weight,
     // softened against itself, no near pairs.  Such a sweep runs like any other
-    // (symmetric matrices, L D L^T, series assembly, shared factors): 21 points
-    // of Ne 1074 in 3 ms instead of 6.3.  Areas that are not the triangles' own
-    // keep the assembly that weighs each RWG side by its own area.
+    // (symmetric matrices, L D L^T, series assembly, shared factors): a call of
+    // 21 points of Ne 1074 takes 3.5 ms instead of 6.5.  Areas that are not the
+    // triangles' own, and meshes of mostly idle triangles, keep the assembly
+    // that weighs each RWG side by its own area.
     CentroidPack cp;
     if (centroid_pack(mesh, p->self_alpha, cp)) {
         o.scheme = EFIE_SCHEME_REF;
