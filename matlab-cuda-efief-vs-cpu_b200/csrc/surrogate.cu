@@ -55,11 +55,13 @@ __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return _
 // (256 CTAs for a layer; 64 x 64 tiles leave half of the SMs idle).  Where 64 x
 // 64 tiles fill it too, each of their operands read from shared memory serves
 // four multiply-adds instead of two.  The sums' order is the same.
+// Four CTAs of the wide tile an SM (64 registers; 78 without the bound, 8 %
+// slower); the narrow one is left to the compiler (58 to 64).
 template <typename TB, int EPI, int T>
-__global__ void __launch_bounds__(GT, 4) k_mlp_gemm(int M, int N, int K, const float *__restrict__ A, long sai,
-                                                 long sak, const TB *__restrict__ B, long sbk, long sbj,
-                                                 float *__restrict__ C, int ldc, const float *__restrict__ bias,
-                                                 float *__restrict__ Aout, int kchunk) {
+__global__ void __launch_bounds__(GT, T == 64 ? 4 : 0)
+    k_mlp_gemm(int M, int N, int K, const float *__restrict__ A, long sai, long sak, const TB *__restrict__ B, long sbk,
+               long sbj, float *__restrict__ C, int ldc, const float *__restrict__ bias, float *__restrict__ Aout,
+               int kchunk) {
     constexpr int R = T / 16, BK = T == 32 ? 32 : 16, PAD = R;   // PAD keeps the rows aligned for R floats
     __shared__ __align__(16) float As[BK][T + PAD];
     __shared__ __align__(16) float Bs[BK][T + PAD];
